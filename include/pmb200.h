@@ -129,11 +129,14 @@ int pmb200_eval(pmb200_ctx *ctx, const double *pos, double *forces,
  * which splits its cells into numberOfBlocks() ranges and evaluates the
  * ranges Parallel::next() grants; Parallel::reduce then sums forces and
  * energies over the ranks, force/ForceGroup.cpp:79-116).  Evaluates on host
- * buffers only the pairs whose i-cell (this library's grid, pmb200_grid) lies
- * in [cell_lo, cell_hi): with the mixed kernel the half-shell pairs of those
- * cells, with the FP64 kernel the forces on their atoms and half their pair
- * energies.  Arguments and accumulation as pmb200_eval; over a partition of
- * [0, number of cells) the shares sum to pmb200_eval's result. */
+ * buffers the share of the pairs that the range [cell_lo, cell_hi) of this
+ * library's cells (pmb200_grid) stands for: in mixed contexts on orthogonal
+ * periodic boxes the same fraction of the column kernels' clusters, otherwise
+ * the pairs whose i-cell lies in the range (with the mixed kernel the
+ * half-shell pairs of those cells, with the FP64 kernel the forces on their
+ * atoms and half their pair energies).  Arguments and accumulation as
+ * pmb200_eval; over a partition of [0, number of cells) the shares sum to
+ * pmb200_eval's result. */
 int pmb200_eval_cells(pmb200_ctx *ctx, const double *pos, double *forces,
                       double *energies, double *virial, double *molvirial,
                       unsigned flags, int cell_lo, int cell_hi);
@@ -175,8 +178,9 @@ int pmb200_autotune(pmb200_ctx *ctx, const double *d_pos, void *stream, int reps
                     double result[8]);
 
 /* The mixed pair kernel of a context.  PMB200_KERNEL_SEARCH (the default):
- * per-atom candidate search in every evaluation (culled staging, per-lane
- * lists).  PMB200_KERNEL_TILES: cluster pairs -- runs of 4 atoms of a cell
+ * a search in every evaluation -- on orthogonal periodic boxes the column
+ * kernels (clusters of 8 atoms against the atoms within the cutoff of their
+ * box), elsewhere per-atom candidate search (culled staging, per-lane lists).  PMB200_KERNEL_TILES: cluster pairs -- runs of 4 atoms of a cell
  * (sorted by height) as clusters, one bounding-box test per cluster pair,
  * and 4 x 4 tiles of atom pairs evaluated with masks; the same pair set and
  * pair arithmetic.  The tile kernel serves the cutoff and real-space Ewald
@@ -205,9 +209,9 @@ int pmb200_set_pair_kernel(pmb200_ctx *ctx, int kernel);
  * (NonbondedCutoffSystemForce::parallelEvaluate, protomol/src/protomol/force/
  * nonbonded/NonbondedCutoffSystemForce.h:57-77, which deals contiguous runs
  * of cell pairs to the ranks and sums the forces with MPI; here contiguous
- * runs of i-cells).  Shard `shard` of `nshards` evaluates the half-shell pairs
- * of the i-cells [ncell * shard / nshards, ncell * (shard + 1) / nshards)
- * into d_facc[3n] (int64, overwritten): the forces in the library's fixed
+ * runs of i-cells, or of the column kernels' clusters).  Shard `shard` of
+ * `nshards` evaluates the pairs of the i-cells (clusters)
+ * [count * shard / nshards, count * (shard + 1) / nshards) into d_facc[3n] (int64, overwritten): the forces in the library's fixed
  * point, an opaque layout whose only use is an element-wise integer sum over
  * the shards (an all-reduce with ncclInt64 / ncclSum, say), exact whatever
  * the reduction order.  d_out[20] (overwritten when flags ask for it)

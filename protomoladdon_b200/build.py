@@ -8,7 +8,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpmb200.so")
-SOURCES = [os.path.join(CSRC, "pmb200_api.cu")]
+SOURCES = [os.path.join(CSRC, f) for f in ("pmb200_api.cu", "pmb200_columns.cu",
+                                                   "pmb200_columns64.cu")]
 DEPS = SOURCES + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + [
     os.path.join(HERE, "..", "include", "pmb200.h")]
 
@@ -17,7 +18,7 @@ DEPS = SOURCES + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fopenmp", "-Xcompiler", "-fno-math-errno",
               "-Xcompiler", "-ffp-contract=off",
-              "-shared", "-cudart", "static",
+              "-shared", "-cudart", "static", "--threads", "0",
               "-lgomp"]
 
 

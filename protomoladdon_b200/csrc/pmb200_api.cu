@@ -11,6 +11,7 @@
 #include "pmb200_kernels.cuh"
 #include "pmb200_tiles.cuh"
 #include "pmb200_clusters.cuh"
+#include "pmb200_columns.h"
 
 #include <algorithm>
 #include <cmath>
@@ -73,6 +74,31 @@ struct pmb200_ctx {
   ScEntry *d_sc_ent = nullptr;
   unsigned long long *d_sc_facc = nullptr;
   double *d_sc_part = nullptr;
+  // column kernels (pmb200_columns.cuh), where they apply (col_ok): the
+  // evaluation path of orthogonal periodic boxes
+  bool col_ok = false, col_full = false;
+  ColGrid cg{};
+  ColStencil cst{};
+  short2 *d_cst = nullptr;    // its classes on the device
+  int col_lsplit = 0;         // log2 of the pair kernel's warps per cluster
+  MixedConsts mcc{};          // the pair constants in the columns' length unit
+  double col_unit = 1.0;      // that unit (A)
+  int col_clusters = 0;       // upper bound of the clusters
+  size_t col_n_alloc = 0, col_slot_alloc = 0, col_ncol_alloc = 0, col_bucket_alloc = 0,
+         col_zs_alloc = 0, col_part_alloc = 0, col_lj_alloc = 0;
+  bool col_count_zero = false;
+  double *d_csq = nullptr;
+  // FP64 kernels: wrapped positions (caller and slot order), a direction
+  double4 *d_dpos = nullptr, *d_cspos64 = nullptr, *d_cw = nullptr;
+  size_t dpos_alloc = 0, cspos64_alloc = 0, cw_alloc = 0;
+  int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr, *d_icom = nullptr;
+  size_t icom_alloc = 0;
+  int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_cscratch = nullptr;
+  int *d_cctl = nullptr;
+  unsigned char *d_ljact = nullptr;
+  float4 *d_ljc32 = nullptr;
+  double2 *d_ljc64 = nullptr;
+  double *d_cpartial = nullptr;
   // tabulated LJ (LennardJonesTableForce under UniversalSwitchingFunction):
   // the FP64 grid on the device (null: analytic LJ)
   double4 *d_ljtab = nullptr;
@@ -407,6 +433,33 @@ int pull_lj(pmb200_ctx *c) {
   return PMB200_OK;
 }
 
+// The column kernels' LJ tables (in their length unit, FP32 and FP64) and, per
+// type, whether any type meets it with a non-zero entry (atoms of the other
+// types -- the hydrogens of 3-site waters -- skip the LJ arithmetic).
+int col_upload_lj(pmb200_ctx *c) {
+  const int nt = c->ntypes, t2 = nt * nt;
+  std::vector<double2> l64(2 * t2);
+  std::vector<float4> l32(t2);
+  std::vector<unsigned char> act(nt, 0);
+  const double u = c->col_unit;
+  const double u6 = std::pow(u, 6.0), u12 = u6 * u6;
+  for (int k = 0; k < t2; k++) {
+    const double *p = &c->h_lj[4 * k];
+    l64[k] = make_double2(p[0] / u12, p[1] / u6);
+    l64[t2 + k] = make_double2(p[2] / u12, p[3] / u6);
+    l32[k] = make_float4((float)l64[k].x, (float)l64[k].y, (float)l64[t2 + k].x,
+                         (float)l64[t2 + k].y);
+    if (p[0] != 0.0 || p[1] != 0.0 || p[2] != 0.0 || p[3] != 0.0) act[k % nt] = 1;
+  }
+  CK(cudaMemcpyAsync(c->d_ljc64, l64.data(), sizeof(double2) * 2 * t2, cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(c->d_ljc32, l32.data(), sizeof(float4) * t2, cudaMemcpyHostToDevice,
+                     c->stream));
+  CK(cudaMemcpyAsync(c->d_ljact, act.data(), (size_t)nt, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return PMB200_OK;
+}
+
 // LJ tables: FP64 in Angstrom units, FP32 in cell units (A / u^12, B / u^6).
 int upload_lj(pmb200_ctx *c) {
   int rc = pull_lj(c);
@@ -427,7 +480,7 @@ int upload_lj(pmb200_ctx *c) {
   CK(cudaMemcpyAsync(c->d_lj32, l32.data(), sizeof(float4) * t2, cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  return PMB200_OK;
+  return c->col_ok ? col_upload_lj(c) : PMB200_OK;
 }
 
 int ensure_atom_buffers(pmb200_ctx *c) {
@@ -618,7 +671,38 @@ int ensure_clear(pmb200_ctx *c, cudaStream_t st) {
     CK(cudaMemsetAsync(c->d_count, 0, sizeof(int) * (size_t)c->g.ncell, st));
     c->count_zero = true;
   }
+  if (c->col_ok && !c->col_count_zero) {
+    CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * (size_t)c->cg.ncol, st));
+    c->col_count_zero = true;
+  }
   return PMB200_OK;
+}
+
+// The FP32 pair constants of the context's potential in the length unit u.
+MixedConsts mixed_consts(const pmb200_ctx *c, double rc, double u) {
+  const pmb200_params &p = c->p;
+  const double rl = p.cutoff_lj / u, ro = p.switchon / u, rq = p.cutoff_coul / u;
+  const double t = rl * rl - ro * ro;
+  MixedConsts m{};
+  m.cut2 = (float)((rc / u) * (rc / u));
+  m.rclj2 = (float)(rl * rl);
+  m.ron2 = (float)(ro * ro);
+  m.rcc2 = (float)(rq * rq);
+  m.s1 = (float)(1.0 / (t * t * t));
+  m.s2 = (float)(rl * rl - 3.0 * ro * ro);
+  m.s3 = (float)(4.0 / (t * t * t));
+  m.c15_1 = (float)(1.5 / rq);
+  m.c05_3 = (float)(0.5 / (rq * rq * rq));
+  m.c15_3 = (float)(1.5 / (rq * rq * rq));
+  m.e15 = 1.5 / rq;
+  m.e05 = 0.5 / (rq * rq * rq);
+  m.csf = (float)c->csf;
+  m.swl = make_switch<float>(c->sw_kind[0], c->sw_par[0], u);
+  m.swc = make_switch<float>(c->sw_kind[1], c->sw_par[1], u);
+  m.ea = (float)(c->ew_alpha * u);
+  m.ea2 = (float)(c->ew_alpha * u * c->ew_alpha * u);
+  m.ea2pi = (float)(2.0 * c->ew_alpha * u / std::sqrt(M_PI));
+  return m;
 }
 
 // Neighbour-cell stencils of the current grid for the cutoff rc: rows (dy,
@@ -937,9 +1021,303 @@ int launch_eval_clusters(pmb200_ctx *c, const double *d_pos, double *d_forces, d
   return PMB200_OK;
 }
 
-// f32 / tail (host-buffer calls of mixed contexts, or null): where the
-// evaluation may put its forces in FP32 and the results with the error flag
-// (k_finalize_reduce); *packed tells whether it did.
+// The FP64 column kernels' buffers (w: and a direction's).
+int col_grow64(pmb200_ctx *c, bool w) {
+  auto grow = [&](double4 *&p, size_t &have, size_t want) -> cudaError_t {
+    if (have >= want && p) return cudaSuccess;
+    have = 0;
+    const cudaError_t e = dalloc(p, want);
+    if (e == cudaSuccess) have = want;
+    return e;
+  };
+  CK(grow(c->d_dpos, c->dpos_alloc, (size_t)c->n));
+  CK(grow(c->d_cspos64, c->cspos64_alloc, c->col_slot_alloc));
+  if (w) CK(grow(c->d_cw, c->cw_alloc, c->col_slot_alloc));
+  return PMB200_OK;
+}
+
+// The column kernels' grid, neighbour columns, constants, tables and buffers
+// for the current box and topology (col_ok = false where they do not apply:
+// general cells and vacuum; the cell kernels then run).
+int col_prepare(pmb200_ctx *c) {
+  c->col_ok = false;
+  if (!c->have_box || !c->have_topo) return PMB200_OK;
+  if (c->g.tric || c->vacuum || c->n <= 0 || c->n >= (1 << 27)) return PMB200_OK;
+  const int n = c->n;
+  const double rc = ctx_rc(c);
+  const double *L = c->g.boxlen;
+  ColGrid g{};
+  // lengths in units of a power-of-two fraction of the x edge (about 4 A): one
+  // quantum is then an exact FP32 number along x, and along y and z in cubes
+  const double u = L[0] / std::exp2(std::max(0.0, std::round(std::log2(L[0] / 4.0))));
+  c->col_unit = u;
+  for (int a = 0; a < 3; a++) {
+    g.boxmin[a] = c->g.boxmin[a];
+    g.edge[a] = L[a];
+    g.inv[a] = 1.0 / L[a];
+    g.qd[a] = L[a] / u / 4294967296.0;
+    g.q[a] = (float)g.qd[a];
+  }
+  // columns about the edge of a cube of kColI atoms wide (measured on water:
+  // 0.9 to 1.15 times that edge within 2%), slabs 0.3 of it high
+  const double rlist = rc * (1.0 + 1e-5);
+  double side = std::cbrt(kColI * L[0] * L[1] * L[2] / n);
+  for (;; side *= 1.25) {
+    g.ncx = std::max(1, std::min(16384, (int)std::lround(L[0] / side)));
+    g.ncy = std::max(1, std::min(16384, (int)std::lround(L[1] / side)));
+    if ((long long)g.ncx * g.ncy > (1 << 22)) continue;
+    const double w[2] = {L[0] / g.ncx, L[1] / g.ncy};
+    // neighbour classes (offsets modulo the grid) by the gap between columns
+    std::vector<std::pair<double, short2>> cls;
+    const int R[2] = {(int)std::ceil(rlist / w[0]), (int)std::ceil(rlist / w[1])};
+    const int nc[2] = {g.ncx, g.ncy};
+    auto gap = [&](int m, int a) {
+      return m == 0 ? 0.0 : std::min(m - 1, nc[a] - m - 1) * w[a];
+    };
+    auto reach = [&](int m, int a) { return std::min(m, nc[a] - m) <= R[a]; };
+    for (int mx = 0; mx < g.ncx; mx++) {
+      if (!reach(mx, 0)) continue;
+      for (int my = 0; my < g.ncy; my++) {
+        if (!reach(my, 1)) continue;
+        const double gx = gap(mx, 0), gy = gap(my, 1);
+        const double d2 = gx * gx + gy * gy;
+        if (d2 > rlist * rlist) continue;
+        const int ox = (g.ncx - mx) % g.ncx, oy = (g.ncy - my) % g.ncy;  // the opposite offset
+        if (std::make_pair(ox, oy) < std::make_pair(mx, my)) continue;   // that one is listed
+        const bool self = ox == mx && oy == my && (mx || my);
+        cls.push_back({d2, make_short2((short)mx, (short)(my | (self ? 0x8000 : 0)))});
+      }
+    }
+    if ((int)cls.size() > kColMaxCls) continue;
+    std::stable_sort(cls.begin(), cls.end(),
+                     [](const auto &x, const auto &y) { return x.first < y.first; });
+    c->cst = ColStencil{};
+    for (const auto &e : cls) c->cst.off[c->cst.n++] = e.second;
+    g.wx = (float)(w[0] / u);
+    g.wy = (float)(w[1] / u);
+    break;
+  }
+  g.ncol = g.ncx * g.ncy;
+  g.nsz = std::max(1, std::min(kColMaxSlabs, (int)std::lround(L[2] / (0.3 * side))));
+  g.cap = (int)std::min<long long>(n, 2LL * n / g.ncol + 64);
+  g.inv_hs = (float)(g.nsz * u / L[2]);
+  g.rc2 = (float)(rlist * rlist / (u * u));
+  g.inv_unit = 1.0 / u;
+  for (int a = 0; a < 3; a++) g.hmax[a] = (float)((0.5 * L[a] - rlist) / u - 1e-3);
+  g.qscale = (float)(1.0 / std::sqrt(u));
+  const long long slots = (long long)n + (long long)(kColI - 1) * g.ncol;
+  g.nslot = (int)((slots + kColI - 1) / kColI * kColI);
+  c->col_clusters = g.nslot / kColI;
+  const int cl = n / kColI;
+  g.nparts = cl >= 16000 ? 1 : (cl >= 2500 ? 2 : (cl >= 600 ? 4 : 8));
+  for (c->col_lsplit = 0; 2 << c->col_lsplit <= g.nparts;) c->col_lsplit++;
+  // buffers
+  auto grow = [&](auto *&p, size_t &have, size_t want) -> cudaError_t {
+    if (have >= want && p) return cudaSuccess;
+    have = 0;
+    const cudaError_t e = dalloc(p, want);
+    if (e == cudaSuccess) have = want;
+    return e;
+  };
+  const size_t t2 = (size_t)c->ntypes * c->ntypes;
+  CK(grow(c->d_ipos, c->col_n_alloc, (size_t)n));
+  if (c->col_slot_alloc < (size_t)g.nslot) {
+    c->col_slot_alloc = 0;
+    CK(dalloc(c->d_cspos, (size_t)g.nslot));
+    CK(dalloc(c->d_csmeta, (size_t)g.nslot));
+    CK(dalloc(c->d_cscratch, (size_t)g.nslot));
+    CK(dalloc(c->d_csq, (size_t)g.nslot));
+    c->col_slot_alloc = (size_t)g.nslot;
+  }
+  CK(grow(c->d_ccount, c->col_ncol_alloc, (size_t)g.ncol));
+  CK(cudaMemset(c->d_ccount, 0, sizeof(int) * (size_t)g.ncol));
+  c->col_count_zero = true;
+  CK(grow(c->d_bucket, c->col_bucket_alloc, (size_t)g.ncol * g.cap));
+  CK(grow(c->d_zs, c->col_zs_alloc, (size_t)g.ncol * (g.nsz + 1)));
+  CK(grow(c->d_cpartial, c->col_part_alloc, (size_t)c->col_clusters * g.nparts * kNacc));
+  CK(grow(c->d_icom, c->icom_alloc, (size_t)std::max(c->nmol, 1)));
+  if (!c->d_cctl) CK(dalloc(c->d_cctl, 4));
+  if (c->p.precision == PMB200_FP64) {  // (mixed contexts: at the first derivative)
+    const int r64 = col_grow64(c, false);
+    if (r64) return r64;
+  }
+  if (!c->d_cst) CK(dalloc(c->d_cst, (size_t)kColMaxCls));
+  CK(cudaMemcpy(c->d_cst, c->cst.off, sizeof(short2) * (size_t)c->cst.n, cudaMemcpyHostToDevice));
+  if (c->col_lj_alloc < t2) {
+    c->col_lj_alloc = 0;
+    CK(dalloc(c->d_ljc32, t2));
+    CK(dalloc(c->d_ljc64, 2 * t2));
+    CK(dalloc(c->d_ljact, (size_t)c->ntypes));
+    c->col_lj_alloc = t2;
+  }
+  c->mcc = mixed_consts(c, rc, u);
+  c->col_full = c->mcc.rclj2 >= c->mcc.cut2 && c->mcc.rcc2 >= c->mcc.cut2;
+  c->cg = g;
+  int r = pull_lj(c);
+  if (r) return r;
+  r = col_upload_lj(c);
+  if (r) return r;
+  c->col_ok = true;
+  release_graph(c);
+  return PMB200_OK;
+}
+
+int prepare_kernels(pmb200_ctx *c) {
+  const int r = col_prepare(c);
+  return r ? r : sc_prepare(c);
+}
+
+// Whether an evaluation runs on the column kernels: where they apply and no
+// other pair kernel was asked for (and serves it).
+bool columns_apply(const pmb200_ctx *c, unsigned flags) {
+  return c->col_ok && c->p.precision == PMB200_MIXED && !clusters_apply(c, flags) &&
+         !tiles_apply(c, flags);
+}
+
+// (d_w: a direction to gather beside the FP64 positions; fp64: these wanted)
+int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
+                     unsigned long long *clear, int nclear = 3, bool fp64 = false,
+                     const double *d_w = nullptr) {
+  const int n = c->n;
+  const ColGrid &g = c->cg;
+  if (fp64) {
+    const int r = col_grow64(c, d_w != nullptr);
+    if (r) return r;
+  }
+  if (!c->col_count_zero)
+    CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * (size_t)g.ncol, st));
+  c->col_count_zero = false;
+  launch_k(k_col_index, (unsigned)((n + 255) / 256), 256, 0, st, false, n, d_pos, g,
+           (const double *)c->d_q, c->d_ipos, c->d_ccount, c->d_bucket, clear,
+           clear ? nclear : 0, c->d_err, fp64 ? c->d_dpos : nullptr);
+  launch_k(k_col_sort, (unsigned)g.ncol, kColSortThreads, 0, st, true, n, g,
+           (const int4 *)c->d_ipos, (const int *)c->d_ccount, (const int *)c->d_bucket,
+           (const int *)c->d_type, (const int *)c->d_mol, (const unsigned char *)c->d_ljact,
+           (const double *)c->d_q, c->d_cspos, c->d_csmeta, c->d_csq, c->d_zs, c->d_cscratch,
+           c->d_cctl, fp64 ? (const double4 *)c->d_dpos : (const double4 *)nullptr,
+           fp64 ? c->d_cspos64 : (double4 *)nullptr, d_w, d_w ? c->d_cw : (double4 *)nullptr);
+  CK(cudaGetLastError());
+  return PMB200_OK;
+}
+
+ColArrays col_arrays(const pmb200_ctx *c) {
+  ColArrays a{};
+  a.spos = c->d_cspos;
+  a.smeta = c->d_csmeta;
+  a.sq = c->d_csq;
+  a.spos64 = c->d_cspos64;
+  a.w = c->d_cw;
+  a.zs = c->d_zs;
+  a.st = c->d_cst;
+  a.st_n = c->cst.n;
+  a.ex_start = c->d_ex_start;
+  a.ex = c->d_ex;
+  a.icom = c->d_icom;
+  a.err = c->d_err;
+  return a;
+}
+
+Col64Launch col64_launch(const pmb200_ctx *c, bool pdl) {
+  Col64Launch l{};
+  l.form = c->form;
+  l.ntypes = c->ntypes;
+  l.full = c->fc.rclj2 >= c->fc.cut2 && c->fc.rcc2 >= c->fc.cut2 && !c->has_modified;
+  l.pdl = pdl;
+  l.lj64 = c->d_lj64;
+  l.acc = c->d_facc;
+  l.ctl = c->d_cctl;
+  l.count = c->d_ccount;
+  l.lsplit = c->col_lsplit;
+  l.clusters = c->col_clusters;
+  l.partial = c->d_cpartial;
+  return l;
+}
+
+// The pair kernel over a share of the clusters.
+int launch_col_pair(pmb200_ctx *c, unsigned flags, cudaStream_t st, bool pdl, ColShare share,
+                    unsigned long long *facc) {
+  ColArrays a = col_arrays(c);
+  a.facc = facc;
+  ColLaunch l{};
+  l.form = c->form;
+  l.ntypes = c->ntypes;
+  l.full = c->col_full;
+  l.mod = c->has_modified;
+  l.molvir = (flags & PMB200_MOLVIRIAL) != 0;
+  l.virial = l.molvir || (flags & PMB200_VIRIAL);
+  l.energy = l.molvir || (flags & PMB200_ENERGY);
+  l.lj32 = c->d_ljc32;
+  l.lj64 = c->d_ljc64;
+  l.ctl = c->d_cctl;
+  l.count = c->d_ccount;
+  l.lsplit = c->col_lsplit;
+  l.share = share;
+  l.clusters = (int)std::min<long long>(
+      c->col_clusters, (long long)c->col_clusters * (share.hi - share.lo) / share.of + 1);
+  l.partial = c->d_cpartial;
+  CK(col_launch_pair(c->cg, c->mcc, a, l, st, pdl));
+  c->col_count_zero = true;  // (the kernel clears the counts)
+  return PMB200_OK;
+}
+
+int launch_eval_columns(pmb200_ctx *c, const double *d_pos, double *d_forces, double *d_out,
+                        unsigned flags, int accumulate, cudaStream_t st, float *f32,
+                        double *tail, bool *packed) {
+  const int n = c->n;
+  const bool energy = (flags & PMB200_ENERGY) != 0;
+  const bool virial = (flags & (PMB200_VIRIAL | PMB200_MOLVIRIAL)) != 0;
+  const bool mixed = c->p.precision == PMB200_MIXED;
+  int r = launch_col_build(c, d_pos, st, c->d_facc, mixed ? 3 : 8, !mixed);
+  if (r) return r;
+  if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
+    k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms, c->d_mass,
+                                                  d_pos, c->d_com);
+    k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(st, &cap));
+  const bool timed = c->timing && cap == cudaStreamCaptureStatusNone;
+  if (timed) CK(cudaEventRecord(c->ev0, st));
+  if (mixed) {
+    r = launch_col_pair(c, flags, st, !timed, ColShare{0, 1, 1}, c->d_facc);
+    if (r) return r;
+  } else {
+    Col64Launch l = col64_launch(c, !timed);
+    l.energy = energy;
+    CK(col_launch_pair64(c->cg, c->fc, col_arrays(c), l, st));
+    c->col_count_zero = true;  // (the kernel clears the counts)
+  }
+  const double scale = kFixInv / c->col_unit;
+  const int ns = virial ? ACC_MV : ACC_E, n3 = 3 * n;
+  const int lsplit = c->col_lsplit;
+  if ((energy || virial) && !timed) {
+    launch_k(mixed ? k_col_finalize_reduce<false> : k_col_finalize_reduce<true>,
+             (unsigned)std::max((n3 + 255) / 256, kRedBlocks), 256, 0, st, true, n,
+             (const unsigned long long *)c->d_facc, scale, accumulate, d_forces,
+             (const int *)c->d_cctl, lsplit, (const double *)c->d_cpartial, c->d_red,
+             c->d_redctr, d_out ? d_out : c->d_out, c->d_pairs, ns, f32, tail,
+             (const int *)c->d_err);
+    if (packed) *packed = tail != nullptr;
+    CK(cudaGetLastError());
+    return PMB200_OK;
+  }
+  launch_k(mixed ? k_col_finalize<false> : k_col_finalize<true>, (unsigned)((n3 + 255) / 256),
+           256, 0, st, !timed, n, (const unsigned long long *)c->d_facc, scale, accumulate,
+           d_forces, (double *)nullptr);
+  if (timed) CK(cudaEventRecord(c->ev1, st));
+  if (energy || virial) {
+    k_col_reduce1<<<kRedBlocks, 256, 0, st>>>(c->d_cctl, lsplit, ColShare{0, 1, 1},
+                                              c->d_cpartial, c->d_red, ns);
+    k_reduce2<<<1, 256, 0, st>>>(kRedBlocks, c->d_red, 1.0, d_out ? d_out : c->d_out,
+                                c->d_pairs, ns);
+  }
+  CK(cudaGetLastError());
+  return PMB200_OK;
+}
+
+// f32 / tail (host-buffer calls, or null): where the evaluation may put its
+// forces in FP32 (mixed contexts) and the results with the error flag; *packed
+// tells whether it did.
 int launch_eval(pmb200_ctx *c, const double *d_pos, double *d_forces, double *d_out,
                 unsigned flags, int accumulate, cudaStream_t st, float *f32 = nullptr,
                 double *tail = nullptr, bool *packed = nullptr) {
@@ -956,6 +1334,9 @@ int launch_eval(pmb200_ctx *c, const double *d_pos, double *d_forces, double *d_
     return launch_eval_clusters(c, d_pos, d_forces, d_out, flags, accumulate, st,
                                 c->timing && cs == cudaStreamCaptureStatusNone);
   }
+  if (columns_apply(c, flags))
+    return launch_eval_columns(c, d_pos, d_forces, d_out, flags, accumulate, st, f32, tail,
+                               packed);
   // the cell build clears the accumulator on the way (still in L2 when the
   // pair kernel adds to it), so that the pair kernel follows the build's last
   // kernel directly
@@ -1247,6 +1628,11 @@ int pmb200_destroy(pmb200_ctx *c) {
   dfree(c->d_sc_clo); dfree(c->d_sc_chi); dfree(c->d_sc_sbox); dfree(c->d_sc_corg);
   dfree(c->d_sc_sorg); dfree(c->d_sc_tasks); dfree(c->d_sc_cmol); dfree(c->d_sc_ent);
   dfree(c->d_sc_facc); dfree(c->d_sc_part);
+  dfree(c->d_ipos); dfree(c->d_cspos); dfree(c->d_csmeta); dfree(c->d_icom);
+  dfree(c->d_ccount); dfree(c->d_bucket); dfree(c->d_zs); dfree(c->d_cscratch);
+  dfree(c->d_cctl); dfree(c->d_ljact); dfree(c->d_ljc32); dfree(c->d_ljc64);
+  dfree(c->d_cpartial); dfree(c->d_csq); dfree(c->d_cst);
+  dfree(c->d_dpos); dfree(c->d_cspos64); dfree(c->d_cw);
   if (c->h_pin_pos) cudaFreeHost(c->h_pin_pos);
   if (c->h_pin_frc) cudaFreeHost(c->h_pin_frc);
   if (c->h_pin_out) cudaFreeHost(c->h_pin_out); dfree(c->d_hpos); dfree(c->d_hfrc);
@@ -1300,7 +1686,9 @@ int pmb200_set_topology(pmb200_ctx *c, int n, const int *type, const double *q_s
   std::vector<std::vector<int2>> per(n);
   bool modified = false;
   for (const auto &kv : kinds) {
-    if (kv.second == 0) continue;
+    // pairs of one molecule only: no pair of two is ever looked up
+    // (OneAtomPairTwo.h:68-80)
+    if (kv.second == 0 || molecule[kv.first.first] != molecule[kv.first.second]) continue;
     modified = modified || kv.second == 1;
     per[kv.first.first].push_back(make_int2(kv.first.second, kv.second));
     per[kv.first.second].push_back(make_int2(kv.first.first, kv.second));
@@ -1361,7 +1749,7 @@ int pmb200_set_topology(pmb200_ctx *c, int n, const int *type, const double *q_s
     return pmb200_set_box(c, c->box_e[0], c->box_e[1], c->box_e[2], c->box_origin);
   if (c->have_box) {
     const int r = upload_lj(c);
-    return r ? r : sc_prepare(c);
+    return r ? r : prepare_kernels(c);
   }
   return PMB200_OK;
 }
@@ -1495,29 +1883,9 @@ int pmb200_set_box(pmb200_ctx *c, const double e1[3], const double e2[3], const 
   }
   // constants
   const pmb200_params &p = c->p;
-  const double u = g.unit;
-  const double rl = p.cutoff_lj / u, ro = p.switchon / u, rq = p.cutoff_coul / u;
-  const double t = rl * rl - ro * ro;
-  MixedConsts &m = c->mc;
-  m.cut2 = (float)((rc / u) * (rc / u));
-  m.rclj2 = (float)(rl * rl);
-  m.ron2 = (float)(ro * ro);
-  m.rcc2 = (float)(rq * rq);
-  m.s1 = (float)(1.0 / (t * t * t));
-  m.s2 = (float)(rl * rl - 3.0 * ro * ro);
-  m.s3 = (float)(4.0 / (t * t * t));
-  m.c15_1 = (float)(1.5 / rq);
-  m.c05_3 = (float)(0.5 / (rq * rq * rq));
-  m.c15_3 = (float)(1.5 / (rq * rq * rq));
-  m.e15 = 1.5 / rq;
-  m.e05 = 0.5 / (rq * rq * rq);
-  m.csf = (float)c->csf;
-  m.ey = (float)(g.edge[1] / u);
-  m.ez = (float)(g.edge[2] / u);
-  m.swl = make_switch<float>(c->sw_kind[0], c->sw_par[0], u);
-  m.swc = make_switch<float>(c->sw_kind[1], c->sw_par[1], u);
-  m.ea = (float)(c->ew_alpha * u);
-  m.ea2pi = (float)(2.0 * c->ew_alpha * u / std::sqrt(M_PI));
+  c->mc = mixed_consts(c, rc, g.unit);
+  c->mc.ey = (float)(g.edge[1] / g.unit);
+  c->mc.ez = (float)(g.edge[2] / g.unit);
   Fp64Consts &f = c->fc;
   const double tl = p.cutoff_lj * p.cutoff_lj - p.switchon * p.switchon;
   f.cut2 = rc * rc;
@@ -1566,7 +1934,7 @@ int pmb200_set_box(pmb200_ctx *c, const double e1[3], const double e2[3], const 
   c->have_box = true;
   if (c->have_topo) {
     const int r = upload_lj(c);
-    return r ? r : sc_prepare(c);
+    return r ? r : prepare_kernels(c);
   }
   return PMB200_OK;
 }
@@ -1636,7 +2004,7 @@ int pmb200_set_pair_kernel(pmb200_ctx *c, int kernel) {
   c->tiles_e = c->tiles_f = kernel == PMB200_KERNEL_TILES;
   c->clu_e = c->clu_f = kernel == PMB200_KERNEL_CLUSTERS;
   release_graph(c);  // graphs hold the previous kernel
-  return sc_prepare(c);
+  return prepare_kernels(c);
 }
 
 int pmb200_autotune(pmb200_ctx *c, const double *d_pos, void *stream, int reps,
@@ -1893,6 +2261,26 @@ int pmb200_shard_eval_device(pmb200_ctx *c, const double *d_pos, int shard, int 
   const int lo = (int)((long long)g.ncell * shard / nshards);
   const int hi = (int)((long long)g.ncell * (shard + 1) / nshards);
   unsigned long long *facc = reinterpret_cast<unsigned long long *>(d_facc);
+  if (c->col_ok) {
+    rc = launch_col_build(c, d_pos, st, facc);
+    if (rc) return rc;
+    if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
+      k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms,
+                                                    c->d_mass, d_pos, c->d_com);
+      k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
+    }
+    const ColShare share{shard, shard + 1, nshards};
+    rc = launch_col_pair(c, flags, st, true, share, facc);
+    if (rc) return rc;
+    if (energy || virial) {
+      const int ns = virial ? ACC_MV : ACC_E;
+      k_col_reduce1<<<kRedBlocks, 256, 0, st>>>(c->d_cctl, c->col_lsplit, share,
+                                                c->d_cpartial, c->d_red, ns);
+      k_reduce2<<<1, 256, 0, st>>>(kRedBlocks, c->d_red, 1.0, d_out, c->d_pairs, ns);
+      CK(cudaGetLastError());
+    }
+    return PMB200_OK;
+  }
   launch_cell_build(c, d_pos, true, energy && c->form == FORM_CUTOFF, st);
   if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0)
     k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms, c->d_mass,
@@ -1932,10 +2320,13 @@ int pmb200_shard_finalize(pmb200_ctx *c, const long long *d_facc, double *d_forc
   if (c->n > 0 && (!d_facc || !d_forces)) return fail(c, PMB200_EINVAL, "null device buffer");
   CK(cudaSetDevice(c->p.device));
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-  if (c->n > 0)
-    k_finalize<<<(c->n + 255) / 256, 256, 0, st>>>(
-        c->n, reinterpret_cast<const unsigned long long *>(d_facc), c->d_sidx,
-        kFixInv / c->g.unit, 1, d_forces);
+  const unsigned long long *facc = reinterpret_cast<const unsigned long long *>(d_facc);
+  if (c->n > 0 && c->col_ok)
+    k_col_finalize<false><<<(3 * c->n + 255) / 256, 256, 0, st>>>(
+        c->n, facc, kFixInv / c->col_unit, 1, d_forces, nullptr);
+  else if (c->n > 0)
+    k_finalize<<<(c->n + 255) / 256, 256, 0, st>>>(c->n, facc, c->d_sidx, kFixInv / c->g.unit, 1,
+                                                  d_forces);
   CK(cudaGetLastError());
   return PMB200_OK;
 }
@@ -1957,7 +2348,9 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
   // a Hessian-vector product asked for neither parameter derivative skips them
   const bool params = mode == DERIV_PARAMS || d_dq || d_dlj;
   const bool half = !params || c->ntypes <= kDerivRegTypes;
-  const int blocks = half ? g.ncell * kDerivSlots : (g.ncell + 3) / 4;
+  const bool col = false;
+  const int blocks = col ? c->col_clusters << c->col_lsplit
+                         : (half ? g.ncell * kDerivSlots : (g.ncell + 3) / 4);
   if (params) {
     if (c->tpart_alloc < (size_t)blocks * nt4) {
       CK(dalloc(c->d_tpart, (size_t)blocks * nt4));
@@ -1977,6 +2370,21 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
       }
       d_dlj = c->d_glj;
     }
+  }
+  if (col) {
+    int r = launch_col_build(c, d_pos, st, c->d_facc, 8, true, mode == DERIV_VJP ? d_w : nullptr);
+    if (r) return r;
+    Col64Launch l = col64_launch(c, true);
+    l.tpart = c->d_tpart;
+    CK(col_launch_deriv64(c->cg, c->fc, col_arrays(c), l, mode, params, st));
+    c->col_count_zero = true;  // (the kernel clears the counts)
+    launch_k(k_col_finalize<true>, (unsigned)((3 * n + 255) / 256), 256, 0, st, true, n,
+             (const unsigned long long *)c->d_facc, 1.0, 0,
+             mode == DERIV_VJP ? d_hv : (double *)nullptr, params ? d_dq : (double *)nullptr);
+    if (params)
+      k_reduce_columns<<<(unsigned)nt4, 1024, 0, st>>>(blocks, (int)nt4, c->d_tpart, d_dlj);
+    CK(cudaGetLastError());
+    return PMB200_OK;
   }
   if (mode == DERIV_VJP && c->ws_alloc < (size_t)std::max(n, 1)) {
     CK(dalloc(c->d_wsorted, (size_t)std::max(n, 1)));
@@ -2016,7 +2424,7 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
           c->d_sidx, c->d_ex_start, c->d_ex, c->d_wsorted, d_hv, d_dq, c->d_tpart);
   }
   if (params && !(half && n == 0))
-    k_reduce_columns<<<(unsigned)nt4, 256, 0, st>>>(blocks, (int)nt4, c->d_tpart, d_dlj);
+    k_reduce_columns<<<(unsigned)nt4, 1024, 0, st>>>(blocks, (int)nt4, c->d_tpart, d_dlj);
   CK(cudaGetLastError());
   return PMB200_OK;
 }
@@ -2089,13 +2497,27 @@ __global__ void k_update_q(int n, const double *__restrict__ src, double *__rest
 
 __global__ void k_update_lj(int t2, const double *__restrict__ src, double u6, double u12,
                             double4 *__restrict__ lj64, float4 *__restrict__ lj32,
-                            int *__restrict__ err) {
+                            int *__restrict__ err, int nt, double v6, double v12,
+                            double2 *__restrict__ ljc64, float4 *__restrict__ ljc32,
+                            unsigned char *__restrict__ act) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= t2) return;
+  if (ljc64 && k < nt) {
+    bool any = false;
+    for (int a = 0; a < nt; a++)
+      for (int e = 0; e < 4; e++) any = any || src[4 * ((size_t)a * nt + k) + e] != 0.0;
+    act[k] = any ? 1 : 0;
+  }
   const double a = src[4 * k], b = src[4 * k + 1], a14 = src[4 * k + 2], b14 = src[4 * k + 3];
   if (!(isfinite(a) && isfinite(b) && isfinite(a14) && isfinite(b14))) atomicOr(err, 4);
   lj64[k] = make_double4(a, b, a14, b14);
   lj32[k] = make_float4((float)(a / u12), (float)(b / u6), (float)(a14 / u12), (float)(b14 / u6));
+  if (ljc64) {  // the column kernels' tables (col_upload_lj)
+    const double2 l = make_double2(a / v12, b / v6), m = make_double2(a14 / v12, b14 / v6);
+    ljc64[k] = l;
+    ljc64[t2 + k] = m;
+    ljc32[k] = make_float4((float)l.x, (float)l.y, (float)m.x, (float)m.y);
+  }
 }
 
 int pmb200_update_params_device(pmb200_ctx *c, const double *d_q_scaled, const double *d_lj,
@@ -2111,8 +2533,11 @@ int pmb200_update_params_device(pmb200_ctx *c, const double *d_q_scaled, const d
   if (d_lj) {
     const int t2 = c->ntypes * c->ntypes;
     const double u6 = std::pow(c->g.unit, 6.0), u12 = u6 * u6;
+    const double v6 = std::pow(c->col_unit, 6.0), v12 = v6 * v6;
     k_update_lj<<<(t2 + 127) / 128, 128, 0, st>>>(t2, d_lj, u6, u12, c->d_lj64, c->d_lj32,
-                                                  c->d_err);
+                                                  c->d_err, c->ntypes, v6, v12,
+                                                  c->col_ok ? c->d_ljc64 : nullptr, c->d_ljc32,
+                                                  c->d_ljact);
     if (!c->ev_lj) CK(cudaEventCreateWithFlags(&c->ev_lj, cudaEventDisableTiming));
     CK(cudaEventRecord(c->ev_lj, st));
     c->lj_dev_newer = true;
@@ -2214,9 +2639,9 @@ int pmb200_eval(pmb200_ctx *c, const double *pos, double *forces, double *energi
       double *tail = reinterpret_cast<double *>(c->d_hf32 + f32_slots);
       bool packed = false;
       int r = launch_eval(c, c->d_hpos, c->d_hfrc, d_hout, flags, 0, st,
-                          f32out ? c->d_hf32 : nullptr, tail, &packed);
+                          f32out ? c->d_hf32 : nullptr, f32out ? tail : d_hout, &packed);
       if (r) return r;
-      if (packed) {
+      if (packed && f32out) {
         e = cudaMemcpyAsync(c->h_pin_frc, c->d_hf32, res32_bytes, cudaMemcpyDeviceToHost, st);
       } else if (f32out) {
         // (the error flag goes into the packed copy's tail)
@@ -2225,7 +2650,7 @@ int pmb200_eval(pmb200_ctx *c, const double *pos, double *forces, double *energi
         if (e == cudaSuccess)
           e = cudaMemcpyAsync(c->h_pin_frc, c->d_hf32, res32_bytes, cudaMemcpyDeviceToHost, st);
       } else {
-        k_copy_word<<<1, 1, 0, st>>>(c->d_err, reinterpret_cast<int *>(d_hout + 20));
+        if (!packed) k_copy_word<<<1, 1, 0, st>>>(c->d_err, reinterpret_cast<int *>(d_hout + 20));
         e = cudaGetLastError();
         if (e == cudaSuccess)
           e = cudaMemcpyAsync(c->h_pin_frc, c->d_hfrc, res_bytes, cudaMemcpyDeviceToHost, st);
@@ -2341,6 +2766,30 @@ int pmb200_eval_cells(pmb200_ctx *c, const double *pos, double *forces, double *
   const bool anyvir = (flags & (PMB200_VIRIAL | PMB200_MOLVIRIAL)) != 0;
   const GridParams &g = c->g;
   const int nc = cell_hi - cell_lo;
+  if (mixed && c->col_ok) {
+    // column kernels: the share of the clusters that the range is of the cells
+    const ColShare share{cell_lo, cell_hi, g.ncell};
+    rc = launch_col_build(c, c->d_hpos, st, c->d_facc);
+    if (rc) return rc;
+    if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
+      k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms,
+                                                    c->d_mass, c->d_hpos, c->d_com);
+      k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
+    }
+    rc = launch_col_pair(c, flags, st, true, share, c->d_facc);
+    if (rc) return rc;
+    k_col_finalize<false><<<(3 * c->n + 255) / 256, 256, 0, st>>>(
+        c->n, c->d_facc, kFixInv / c->col_unit, 0, c->d_hfrc, nullptr);
+    if (energy || anyvir) {
+      const int ns = anyvir ? ACC_MV : ACC_E;
+      k_col_reduce1<<<kRedBlocks, 256, 0, st>>>(c->d_cctl, c->col_lsplit, share, c->d_cpartial,
+                                                c->d_red, ns);
+      k_reduce2<<<1, 256, 0, st>>>(kRedBlocks, c->d_red, 1.0, c->d_out, c->d_pairs, ns);
+      CK(cudaMemcpyAsync(c->h_pin_out, c->d_out, sizeof(double) * 20, cudaMemcpyDeviceToHost,
+                         st));
+    }
+    CK(cudaGetLastError());
+  } else {
   launch_cell_build(c, c->d_hpos, mixed, mixed && energy && c->form == FORM_CUTOFF, st,
                     mixed ? c->d_facc : nullptr);
   if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0)
@@ -2378,6 +2827,7 @@ int pmb200_eval_cells(pmb200_ctx *c, const double *pos, double *forces, double *
                                 c->d_pairs, ns);
     CK(cudaMemcpyAsync(c->h_pin_out, c->d_out, sizeof(double) * 20, cudaMemcpyDeviceToHost,
                        st));
+  }
   }
   CK(cudaMemcpyAsync(c->h_pin_frc, c->d_hfrc, bytes, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -3072,6 +3522,20 @@ struct pmb200_batch {
   double *d_partial = nullptr, *d_pairs = nullptr, *d_scratch_f = nullptr;
   int4 *d_tasks = nullptr;
   int *d_rows_start = nullptr, *d_rows = nullptr;
+  // column kernels (every system periodic and orthogonal)
+  bool col = false, col_full = true, col_mod = false, col_dirty = false;
+  std::vector<ColBatchSys> h_col;
+  std::vector<int> col_parts;   // each context's own number of parts
+  int ncol = 0;
+  ColBatchSys *d_col = nullptr;
+  int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_scratch = nullptr;
+  int *d_ctl = nullptr, *d_col_sys = nullptr;
+  int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr;
+  double *d_csq = nullptr;
+  short2 *d_cst = nullptr;
+  unsigned char *d_ljact = nullptr;
+  float4 *d_ljc32 = nullptr;
+  double2 *d_ljc64 = nullptr;
   // schedule: stencil parts per cell, task order (0 as built, 1 by cost,
   // largest first), persistent blocks per SM
   int parts = 1, order = 1, bpsm = 0, max_bpsm = 1, nsm = 1;
@@ -3120,7 +3584,21 @@ void batch_release_graph(pmb200_batch *b) {
 int batch_build_tasks(pmb200_batch *b) {
   std::vector<int4> tasks;
   tasks.reserve((size_t)b->C * b->parts);
-  for (int s = 0; s < b->nsys; s++)
+  if (b->col) {
+    // column kernels: one task per cluster (their upper bound) and part.  Four
+    // parts: dealt as each context deals its own, so that the forces are the
+    // contexts' bit for bit (FP32 sums are grouped by part)
+    for (int s = 0; s < b->nsys; s++) {
+      ColGrid &g = b->h_col[s].g;
+      g.nparts = b->parts == 4 ? b->col_parts[s] : b->parts;
+      const int warps = std::min(b->parts, g.nparts);
+      for (int c = 0; c < g.nslot / kColI; c++)
+        for (int p = 0; p < warps; p++) tasks.push_back(make_int4(s, c, p, warps));
+    }
+    BCK(cudaMemcpy(b->d_col, b->h_col.data(), sizeof(ColBatchSys) * b->nsys,
+                   cudaMemcpyHostToDevice));
+  }
+  for (int s = 0; s < b->nsys && !b->col; s++)
     for (int c = 0; c < b->h_sys[s].g.ncell; c++)
       for (int p = 0; p < b->parts; p++) tasks.push_back(make_int4(s, c, p, b->parts));
   if (b->order == 1)
@@ -3165,6 +3643,37 @@ void batch_launch_pair(pmb200_batch *b, bool energy, bool virial, int grid, cuda
 #undef PMB_BATCH_LAUNCH
 }
 
+ColBatchLaunch batch_col_launch(const pmb200_batch *b, bool energy, bool virial, ColArrays &a) {
+  a = ColArrays{};
+  a.spos = b->d_cspos;
+  a.smeta = b->d_csmeta;
+  a.sq = b->d_csq;
+  a.zs = b->d_zs;
+  a.ex_start = b->d_ex_start;
+  a.ex = b->d_ex;
+  a.facc = b->d_facc;
+  a.err = b->d_err;
+  ColBatchLaunch l{};
+  l.form = b->form;
+  l.full = b->col_full;
+  l.mod = b->col_mod;
+  l.energy = energy;
+  l.virial = virial;
+  l.sys = b->d_col;
+  l.tasks = b->d_tasks;
+  l.ntasks = b->ntasks;
+  l.counter = b->d_counter;
+  l.st = b->d_cst;
+  l.lj32 = b->d_ljc32;
+  l.lj64 = b->d_ljc64;
+  l.ctl = b->d_ctl;
+  l.count = b->d_ccount;
+  l.ncol = b->ncol;
+  l.lj_max = b->lj_max;
+  l.partial = b->d_partial;
+  return l;
+}
+
 // One evaluation of every system on `st` (forces accumulated into d_forces,
 // or overwritten when accumulate is 0).
 int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, double *d_out,
@@ -3174,6 +3683,34 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
   const bool virial = (flags & PMB200_VIRIAL) != 0;
   // the FP32 coordinates' residuals feed the cutoff form's energy sums
   const bool lo = energy && b->form == FORM_CUTOFF;
+  if (b->col) {
+    // (a sequence that broke off leaves its counts behind)
+    if (b->col_dirty) BCK(cudaMemsetAsync(b->d_ccount, 0, sizeof(int) * (size_t)b->ncol, st));
+    b->col_dirty = true;
+    k_col_index_batch<<<(N + 255) / 256, 256, 0, st>>>(N, d_pos, b->d_col, b->d_atom_sys, b->d_q,
+                                                       b->d_ipos, b->d_ccount, b->d_bucket,
+                                                       b->d_facc, b->d_err);
+    k_col_sort_batch<<<b->ncol, kColSortThreads, 0, st>>>(
+        b->d_col, b->d_col_sys, b->d_ipos, b->d_ccount, b->d_bucket, b->d_type, b->d_mol,
+        b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_zs, b->d_scratch, b->d_ctl);
+    BCK(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
+    ColArrays a{};
+    ColBatchLaunch l = batch_col_launch(b, energy, virial, a);
+    const int fit = b->occ[(energy ? 1 : 0) | (virial ? 2 : 0)];
+    const int bpsm = b->bpsm > 0 ? std::min(b->bpsm, fit) : fit;
+    l.grid = std::max(1, std::min(b->ntasks, bpsm * b->nsm));
+    if (timed) BCK(cudaEventRecord(b->ev0, st));
+    BCK(col_launch_batch(a, l, st, nullptr));
+    b->col_dirty = false;  // (the kernel clears the counts)
+    if (timed) BCK(cudaEventRecord(b->ev1, st));
+    k_col_finalize_batch<<<(3 * N + 255) / 256, 256, 0, st>>>(N, b->d_facc, b->d_atom_sys,
+                                                              b->d_col, accumulate, d_forces);
+    if ((energy || virial) && d_out)
+      k_reduce_batch<<<b->nsys, 128, 0, st>>>(b->d_rows_start, b->d_rows, b->d_partial, d_out,
+                                               b->d_pairs, virial ? ACC_MV : ACC_E);
+    BCK(cudaGetLastError());
+    return PMB200_OK;
+  }
   BCK(cudaMemsetAsync(b->d_count, 0, sizeof(int) * b->C, st));
   if (N > 0)
     k_cell_index_batch<<<(N + 255) / 256, 256, 0, st>>>(N, d_pos, b->d_sys, b->d_atom_sys,
@@ -3206,10 +3743,92 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
     k_finalize_batch<<<(N + 255) / 256, 256, 0, st>>>(N, b->d_facc, b->d_sidx, b->d_atom_sys,
                                                       b->d_sys, accumulate, d_forces);
   if ((energy || virial) && d_out)
-    k_reduce_batch<<<(b->nsys + 3) / 4, 128, 0, st>>>(b->nsys, b->d_rows_start, b->d_rows,
-                                                       b->d_partial, b->d_sys, d_out, b->d_pairs,
-                                                       virial ? ACC_MV : ACC_E);
+    k_reduce_batch<<<b->nsys, 128, 0, st>>>(b->d_rows_start, b->d_rows, b->d_partial, d_out,
+                                             b->d_pairs, virial ? ACC_MV : ACC_E);
   BCK(cudaGetLastError());
+  return PMB200_OK;
+}
+
+// The column kernels' layout of a batch: every system's columns, slots, buckets,
+// slab tables, classes and LJ tables back to back.
+int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
+  std::vector<short2> cls;
+  std::vector<int> col_sys;
+  std::vector<float4> l32;
+  std::vector<double2> l64;
+  std::vector<unsigned char> act;
+  long long slots = 0, zs = 0, bucket = 0;
+  for (int s = 0; s < b->nsys; s++) {
+    pmb200_ctx *c = systems[s];
+    ColBatchSys y{};
+    y.atom0 = b->h_sys[s].atom0;
+    y.natoms = c->n;
+    y.col0 = (int)col_sys.size();
+    y.slot0 = (int)slots;
+    y.zs0 = (int)zs;
+    y.bucket0 = (int)bucket;
+    y.st0 = (int)cls.size();
+    y.lj0 = (int)l32.size();
+    y.act0 = (int)act.size();
+    y.ntypes = c->ntypes;
+    b->col_parts.push_back(1);
+    if (c->n > 0) {
+      y.g = c->cg;
+      y.mc = c->mcc;
+      y.fscale = kFixInv / c->col_unit;
+      y.st_n = c->cst.n;
+      cls.insert(cls.end(), c->cst.off, c->cst.off + c->cst.n);
+      col_sys.insert(col_sys.end(), c->cg.ncol, s);
+      b->col_parts.back() = c->cg.nparts;
+      b->col_full = b->col_full && c->col_full;
+      b->col_mod = b->col_mod || c->has_modified;
+      const size_t t2 = (size_t)c->ntypes * c->ntypes;
+      l32.resize(l32.size() + t2);
+      l64.resize(l64.size() + 2 * t2);
+      act.resize(act.size() + c->ntypes);
+      BCK(cudaMemcpy(&l32[y.lj0], c->d_ljc32, sizeof(float4) * t2, cudaMemcpyDeviceToHost));
+      BCK(cudaMemcpy(&l64[2 * (size_t)y.lj0], c->d_ljc64, sizeof(double2) * 2 * t2,
+                     cudaMemcpyDeviceToHost));
+      BCK(cudaMemcpy(&act[y.act0], c->d_ljact, (size_t)c->ntypes, cudaMemcpyDeviceToHost));
+      slots += c->cg.nslot;
+      zs += (long long)c->cg.ncol * (c->cg.nsz + 1);
+      bucket += (long long)c->cg.ncol * c->cg.cap;
+      const double vol = c->g.boxlen[0] * c->g.boxlen[1] * c->g.boxlen[2];
+      b->cost[s] = c->n / vol * std::pow(ctx_rc(c), 3.0);
+    }
+    b->h_col.push_back(y);
+  }
+  if (slots > (1LL << 30) || zs > (1LL << 30) || bucket > (1LL << 30)) {
+    b->col = false;  // (the cell kernels take it)
+    return PMB200_OK;
+  }
+  b->ncol = (int)col_sys.size();
+  const size_t N = (size_t)std::max(b->N, 1), S = (size_t)slots;
+  BCK(dalloc(b->d_col, (size_t)b->nsys));
+  BCK(dalloc(b->d_ccount, col_sys.size()));
+  BCK(cudaMemset(b->d_ccount, 0, sizeof(int) * col_sys.size()));
+  BCK(dalloc(b->d_bucket, (size_t)bucket));
+  BCK(dalloc(b->d_zs, (size_t)zs));
+  BCK(dalloc(b->d_scratch, S));
+  BCK(dalloc(b->d_ctl, (size_t)b->nsys));
+  BCK(cudaMemset(b->d_ctl, 0, sizeof(int) * (size_t)b->nsys));
+  BCK(dalloc(b->d_col_sys, col_sys.size()));
+  BCK(dalloc(b->d_ipos, N));
+  BCK(dalloc(b->d_cspos, S));
+  BCK(dalloc(b->d_csmeta, S));
+  BCK(dalloc(b->d_csq, S));
+  BCK(dalloc(b->d_cst, cls.size()));
+  BCK(dalloc(b->d_ljact, act.size()));
+  BCK(dalloc(b->d_ljc32, l32.size()));
+  BCK(dalloc(b->d_ljc64, l64.size()));
+  auto up = [&](auto *dst, const auto &v) {
+    return cudaMemcpy(dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+  };
+  BCK(up(b->d_col_sys, col_sys));
+  BCK(up(b->d_cst, cls));
+  BCK(up(b->d_ljact, act));
+  BCK(up(b->d_ljc32, l32));
+  BCK(up(b->d_ljc64, l64));
   return PMB200_OK;
 }
 
@@ -3228,6 +3847,9 @@ int pmb200_batch_destroy(pmb200_batch *b) {
   dfree(b->d_rel32); dfree(b->d_spos32); dfree(b->d_rel_lo); dfree(b->d_spos_lo); dfree(b->d_smeta); dfree(b->d_facc);
   dfree(b->d_partial); dfree(b->d_pairs); dfree(b->d_scratch_f); dfree(b->d_tasks);
   dfree(b->d_rows_start); dfree(b->d_rows);
+  dfree(b->d_col); dfree(b->d_ccount); dfree(b->d_bucket); dfree(b->d_zs); dfree(b->d_scratch);
+  dfree(b->d_ctl); dfree(b->d_col_sys); dfree(b->d_ipos); dfree(b->d_cspos); dfree(b->d_csmeta);
+  dfree(b->d_csq); dfree(b->d_cst); dfree(b->d_ljact); dfree(b->d_ljc32); dfree(b->d_ljc64);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   delete b;
@@ -3379,8 +4001,23 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
     cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel, 32, b->smem));
     out = std::max(1, o);
   };
+  // the column kernels' part (systems that all take them)
+  b->col = N > 0;
+  for (int s = 0; s < nsys; s++) b->col = b->col && (systems[s]->col_ok || systems[s]->n == 0);
+  if (b->col) {
+    rc = batch_create_columns(b, systems);
+    if (rc) return done(rc);
+    for (int v = 0; v < 4; v++) {
+      ColArrays a{};
+      const ColBatchLaunch l = batch_col_launch(b, v & 1, v & 2, a);
+      int o = 1;
+      cuda(col_launch_batch(a, l, nullptr, &o));
+      b->occ[v] = std::max(1, o);
+    }
+  }
   // per (energy, virial) variant of the batch's form
-  if (b->form == FORM_GENERIC) {
+  if (b->col) {
+  } else if (b->form == FORM_GENERIC) {
     fits(k_pair_mixed_batch<FORM_GENERIC, false, false>, b->occ[0]);
     fits(k_pair_mixed_batch<FORM_GENERIC, true, false>, b->occ[1]);
     fits(k_pair_mixed_batch<FORM_GENERIC, false, true>, b->occ[2]);

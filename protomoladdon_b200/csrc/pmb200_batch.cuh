@@ -61,7 +61,7 @@ __global__ void k_cell_index_batch(int N, const double *__restrict__ pos,
 // changes.  Dynamic shared memory: lj_max float4 LJ records, then st_max
 // stencil offsets (the largest of any system in the batch).
 template <int kForm, bool kEnergy, bool kVirial>
-__global__ void __launch_bounds__(32, (kEnergy || kVirial) ? 1 : 24)
+__global__ void __launch_bounds__(32, kVirial ? 8 : (kEnergy ? PMB200_ENERGY_BLOCKS : 24))
 k_pair_mixed_batch(const BatchSys *__restrict__ sys, const int4 *__restrict__ tasks, int ntasks,
                    int *__restrict__ counter, const unsigned short *__restrict__ stencils,
                    const float4 *__restrict__ lj32, const int *__restrict__ start,
@@ -126,24 +126,35 @@ __global__ void k_finalize_batch(int N, const unsigned long long *__restrict__ f
   }
 }
 
-// One warp per system: its task rows summed in list order (deterministic),
-// then the same outputs as k_reduce2 (out[s][20]: COULOMB, LENNARDJONES,
-// virial 9, molecular virial 9 (zero)); pairs[s] = in-cutoff pair count.
-__global__ void k_reduce_batch(int nsys, const int *__restrict__ rows_start,
-                               const int *__restrict__ rows, const double *__restrict__ partial,
-                               const BatchSys *__restrict__ sys, double *__restrict__ out,
-                               double *__restrict__ pairs, int ns) {
-  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (s >= nsys) return;
-  double acc = 0.0;  // lane k < ns sums slot k (the slots the launch filled; the rest 0)
-  if (lane < ns)
-    for (int r = rows_start[s]; r < rows_start[s + 1]; r++)
-      acc += partial[(size_t)rows[r] * kNacc + lane];
+// One block of 128 threads per system: its task rows summed in list order by
+// thread, then by a fixed tree (deterministic), then the same outputs as
+// k_reduce2 (out[s][20]: COULOMB, LENNARDJONES, virial 9, molecular virial 9
+// (zero)); pairs[s] = in-cutoff pair count.  (One warp per system, its rows one
+// after another, took 73 us on 512 boxes: the largest has some thousand rows.)
+static __global__ void __launch_bounds__(128)
+k_reduce_batch(const int *__restrict__ rows_start, const int *__restrict__ rows,
+               const double *__restrict__ partial, double *__restrict__ out,
+               double *__restrict__ pairs, int ns) {
+  __shared__ double sh[4][ACC_MV];
+  const int s = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
   double v[ACC_MV];
 #pragma unroll
-  for (int k = 0; k < ACC_MV; k++) v[k] = __shfl_sync(0xffffffffu, acc, k);
-  if (lane != 0) return;
+  for (int k = 0; k < ACC_MV; k++) v[k] = 0.0;
+  for (int r = rows_start[s] + t; r < rows_start[s + 1]; r += 128) {
+    const double *row = partial + (size_t)rows[r] * kNacc;
+#pragma unroll
+    for (int k = 0; k < ACC_MV; k++)
+      if (k < ns) v[k] += row[k];
+  }
+#pragma unroll
+  for (int k = 0; k < ACC_MV; k++) {
+    const double sum = k < ns ? warp_sum_mask(v[k], 32) : 0.0;
+    if (lane == 0) sh[w][k] = sum;
+  }
+  __syncthreads();
+  if (t != 0) return;
+#pragma unroll
+  for (int k = 0; k < ACC_MV; k++) v[k] = sh[0][k] + sh[1][k] + sh[2][k] + sh[3][k];
   double *o = out + 20 * (size_t)s;
   o[0] = v[ACC_ECOUL];
   o[1] = v[ACC_ELJ];

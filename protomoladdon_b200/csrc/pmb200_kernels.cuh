@@ -219,7 +219,7 @@ struct MixedConsts {   // FP32 constants in cell units
   float csf;                 // coulombScalingFactor
   float ey, ez;              // edge[1] / unit, edge[2] / unit (1 for cubic cells)
   double e15, e05;           // C1 energy (FP64): 1.5 / rc_coul and 0.5 / rc_coul^3 (cell units)
-  float ea, ea2pi;           // Ewald alpha and 2 alpha / sqrt(pi), per cell unit
+  float ea, ea2, ea2pi;      // Ewald alpha, its square, 2 alpha / sqrt(pi), per cell unit
   SwitchSpec<float> swl, swc;  // generic form: LJ and Coulomb switches
 };
 
@@ -341,7 +341,7 @@ __device__ __forceinline__ bool locate_cell(const double *xin, const GridParams 
 }
 
 // clear: an accumulator of nclear x n entries zeroed on the way (or null).
-__global__ void k_cell_index(int n, const double *__restrict__ pos, GridParams g,
+static __global__ void k_cell_index(int n, const double *__restrict__ pos, GridParams g,
                              int *__restrict__ cell_of, int *__restrict__ cell_count,
                              int *__restrict__ slot, float4 *__restrict__ rel32,
                              double4 *__restrict__ rel64, const double *__restrict__ q,
@@ -376,7 +376,7 @@ __global__ void k_cell_index(int n, const double *__restrict__ pos, GridParams g
 // Exclusive scan of cell counts in one block (C is a few thousand to a few
 // hundred thousand cells; each thread scans a contiguous span).
 // (the counts are cleared once read, ready for the next build's atomics)
-__global__ void k_scan(int ncell, int *__restrict__ count, int *__restrict__ start) {
+static __global__ void k_scan(int ncell, int *__restrict__ count, int *__restrict__ start) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ int sh[];
@@ -418,7 +418,7 @@ __global__ void k_scan(int ncell, int *__restrict__ count, int *__restrict__ sta
   if (t == T - 1) start[ncell] = incl;
 }
 
-__global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__restrict__ slot,
+static __global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__restrict__ slot,
                           const int *__restrict__ start, int *__restrict__ tmp) {
   pdl_trigger();
   pdl_wait();
@@ -430,7 +430,7 @@ __global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__r
 // One warp per cell: order the cell's atoms by original index (rank = number
 // of members with a smaller index) and gather their data to sorted positions,
 // so the layout, and every sum over it, is the same on every run.
-__global__ void k_rank_gather(int ncell, const int *__restrict__ start,
+static __global__ void k_rank_gather(int ncell, const int *__restrict__ start,
                               const int *__restrict__ tmp, const float4 *__restrict__ rel32,
                               const double4 *__restrict__ rel64, const int *__restrict__ type,
                               const int *__restrict__ mol, int *__restrict__ sidx,
@@ -1286,7 +1286,7 @@ inline size_t mixed_smem_bytes(int form, int ntypes, int st_ncells) {
 // Fixed-point force accumulator (sorted order, [3][n], 2^-32 quanta in cell
 // units) -> FP64 forces in the caller's atom order, accumulated or
 // overwritten.
-__global__ void k_finalize(int n, const unsigned long long *__restrict__ facc,
+static __global__ void k_finalize(int n, const unsigned long long *__restrict__ facc,
                            const int *__restrict__ sidx, double scale, int accumulate,
                            double *__restrict__ forces) {
   pdl_wait();
@@ -1747,7 +1747,7 @@ k_pair_fp64_half(GridParams g, Fp64Consts mc, const HalfStencil st, int slots, i
 
 // The FP64 half-shell kernel's accumulator (sorted order, fix2 words
 // [6][n]) -> forces in the caller's atom order, accumulated or overwritten.
-__global__ void k_finalize64(int n, const unsigned long long *__restrict__ acc,
+static __global__ void k_finalize64(int n, const unsigned long long *__restrict__ acc,
                              const int *__restrict__ sidx, int accumulate,
                              double *__restrict__ forces) {
   pdl_wait();
@@ -2264,7 +2264,7 @@ k_deriv_fp64_half(GridParams g, Fp64Consts mc, const HalfStencil st, int slots, 
 
 // dq from the derivative accumulator's words {hi, lo} (rows 6, 7), in the
 // caller's atom order.
-__global__ void k_finalize_q(int n, const unsigned long long *__restrict__ acc,
+static __global__ void k_finalize_q(int n, const unsigned long long *__restrict__ acc,
                              const int *__restrict__ sidx, double *__restrict__ dq) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
@@ -2275,7 +2275,7 @@ __global__ void k_finalize_q(int n, const unsigned long long *__restrict__ acc,
 
 // ws[j] = w[3 sidx[j] ..] for the sorted atoms j (the direction of a
 // Hessian-vector product, read per pair in cell order).
-__global__ void k_gather_sorted(int n, const int *__restrict__ sidx, const double *__restrict__ w,
+static __global__ void k_gather_sorted(int n, const int *__restrict__ sidx, const double *__restrict__ w,
                                 double4 *__restrict__ ws) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
@@ -2283,24 +2283,29 @@ __global__ void k_gather_sorted(int n, const int *__restrict__ sidx, const doubl
   ws[j] = make_double4(w[o], w[o + 1], w[o + 2], 0.0);
 }
 
-// out[k] = sum over rows r of part[r][k], rows added in order (deterministic).
-__global__ void k_reduce_columns(int rows, int cols, const double *__restrict__ part,
-                                 double *__restrict__ out) {
-  // one block per column (part[col][row]): strided per-thread sums, then a
-  // fixed tree, so the order of the additions is the same every launch
-  __shared__ double red[256];
-  const int k = blockIdx.x;
+// out[k] = sum over rows r of part[k][r], one block of 1024 threads per column:
+// four strided sums per thread, then a fixed tree, so the order of the additions
+// is the same every launch.  (256 threads adding 43 rows each, one load after
+// another, took 23 us on the 11k rows of the 41k-atom box.)
+static __global__ void __launch_bounds__(1024)
+k_reduce_columns(int rows, int cols, const double *__restrict__ part,
+                 double *__restrict__ out) {
+  __shared__ double red[32];
+  const int k = blockIdx.x, t = threadIdx.x;
   if (k >= cols) return;
   const double *col = part + (size_t)k * rows;
-  double acc = 0.0;
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) acc += col[r];
-  red[threadIdx.x] = acc;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int r = t; r < rows; r += 4096)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (r + 1024 * q < rows) a[q] += col[r + 1024 * q];
+  const double s = warp_sum_mask((a[0] + a[1]) + (a[2] + a[3]), 32);
+  if ((t & 31) == 0) red[t >> 5] = s;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (t < 32) {
+    const double v = warp_sum_mask(red[t], 32);
+    if (t == 0) out[k] = v;
   }
-  if (threadIdx.x == 0) out[k] = red[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -2308,7 +2313,7 @@ __global__ void k_reduce_columns(int rows, int cols, const double *__restrict__ 
 // (mass-weighted, Kahan-compensated like molecularCenterOfMass,
 // protomol/src/protomol/topology/TopologyUtilities.cpp:645-672).
 // ---------------------------------------------------------------------------
-__global__ void k_com(int nmol, const int *__restrict__ mstart, const int *__restrict__ matoms,
+static __global__ void k_com(int nmol, const int *__restrict__ mstart, const int *__restrict__ matoms,
                       const double *__restrict__ mass, const double *__restrict__ pos,
                       double *__restrict__ com) {
   int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2411,14 +2416,14 @@ __device__ __forceinline__ void reduce2_block(int nred, const double *red, doubl
 }
 
 // Launched with kRedBlocks blocks of 256 threads.
-__global__ void k_reduce1(int nrows, const double *__restrict__ partial,
+static __global__ void k_reduce1(int nrows, const double *__restrict__ partial,
                           double *__restrict__ red, int ns) {
   __shared__ double sh[8][ACC_MV];
   reduce1_block(blockIdx.x, nrows, partial, red, ns, sh);
 }
 
 // One block of 256 threads; nred = kRedBlocks.
-__global__ void k_reduce2(int nred, const double *__restrict__ red, double visit,
+static __global__ void k_reduce2(int nred, const double *__restrict__ red, double visit,
                           double *__restrict__ out, double *__restrict__ pairs_out, int ns) {
   __shared__ double col[ACC_MV];
   reduce2_block(nred, red, visit, out, pairs_out, ns, col);
@@ -2436,7 +2441,7 @@ __global__ void k_reduce2(int nred, const double *__restrict__ red, double visit
 // there in FP32 (the FP64 values rounded once) instead of to `forces`, and
 // the 20 result words and the device error flag `err` to `tail` after them,
 // for one copy back to the host.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
 k_finalize_reduce(int n, const unsigned long long *__restrict__ facc,
                   const int *__restrict__ sidx, double scale, int accumulate,
                   double *__restrict__ forces, int nrows, const double *__restrict__ partial,
@@ -2482,7 +2487,7 @@ k_finalize_reduce(int n, const unsigned long long *__restrict__ facc,
 // Leapfrog kick + drift (LeapfrogIntegrator::doKickdoDrift without modifiers,
 // protomol/src/protomol/integrator/leapfrog/LeapfrogIntegrator.cpp:72-85):
 // v += F * kick / m; x += v * h.  drift == 0 gives a kick only.
-__global__ void k_kick_drift(int n, double *__restrict__ pos, double *__restrict__ vel,
+static __global__ void k_kick_drift(int n, double *__restrict__ pos, double *__restrict__ vel,
                              const double *__restrict__ frc, const double *__restrict__ mass,
                              double kick, double h, int drift) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2518,7 +2523,7 @@ __device__ __forceinline__ void d_unit(double a[3]) {
 }
 
 // old: A0 B0 C0 (constrained); in/out: A1 B1 C1 (unconstrained -> constrained)
-__device__ void settle_water(const SettleParams &sp, const double *A0, const double *B0,
+static __device__ void settle_water(const SettleParams &sp, const double *A0, const double *B0,
                              const double *C0, double *A1, double *B1, double *C1) {
   const double M = sp.mo + 2.0 * sp.mh;
   double com[3], a1[3], b1[3], c1[3], b0[3], c0[3], ex[3], ey[3], ez[3];
@@ -2561,7 +2566,7 @@ __device__ void settle_water(const SettleParams &sp, const double *A0, const dou
 
 // Kick + drift with rigid waters: unit u < nwater is a water (one thread:
 // kick, drift, SETTLE, v = (x_new - x_old) / h); the rest are free atoms.
-__global__ void k_kick_drift_settle(int nwater, const int *__restrict__ widx, int nfree,
+static __global__ void k_kick_drift_settle(int nwater, const int *__restrict__ widx, int nfree,
                                     const int *__restrict__ fidx, double *__restrict__ pos,
                                     double *__restrict__ vel, const double *__restrict__ frc,
                                     const double *__restrict__ mass, double kick, double h,
@@ -2598,7 +2603,7 @@ __global__ void k_kick_drift_settle(int nwater, const int *__restrict__ widx, in
 }
 
 // FP32 FMA throughput probe: 8 independent FMA chains per thread.
-__global__ void k_fma_peak(int iters, float seed, float *__restrict__ sink) {
+static __global__ void k_fma_peak(int iters, float seed, float *__restrict__ sink) {
   float a0 = seed + threadIdx.x, a1 = a0 + 1.f, a2 = a0 + 2.f, a3 = a0 + 3.f;
   float a4 = a0 + 4.f, a5 = a0 + 5.f, a6 = a0 + 6.f, a7 = a0 + 7.f;
   const float m = 0.999999f, b = 1e-7f;

@@ -1,0 +1,108 @@
+"""The column kernels (the evaluation path of orthogonal periodic boxes) at the
+shapes where their layout has edges: clusters of 8 atoms and blocks of 32 staged
+ones that do not fill, boxes of exactly two cutoffs, columns that are their own
+opposite, columns whose atoms overflow their bucket or the sort's shared memory,
+clusters taller than the cutoff, exclusion lists longer than a warp -- against
+the FP64 oracle.
+
+Tolerances: forces 1e-5 RMS relative (the mixed kernels' bound; FP32 pair
+arithmetic leaves about 1e-6); energies 1e-6 of the pair magnitudes, about
+100 kcal/mol per atom; the pair set is the oracle's up to one pair in 1e6 at the
+cutoff."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from protomoladdon_b200 import water
+from protomoladdon_b200.force import (NonbondedCutoffB200SystemForce, PeriodicTopology,
+                                      ScalarStructure)
+
+pytestmark = pytest.mark.gpu
+
+
+def _waters(n, edges, region=None, seed=3, rc=8.0):
+    """n waters in a box of the given edges, on a jittered lattice filling
+    `region` (the whole box by default) at most as densely as water."""
+    edges = np.asarray(edges, dtype=np.float64)
+    region = edges if region is None else np.asarray(region, dtype=np.float64)
+    k = np.maximum(1, np.floor(region / (np.prod(region) / n) ** (1 / 3.0)).astype(int))
+    while np.prod(k) < n:
+        k[np.argmax(region / k)] += 1
+    rng = np.random.default_rng(seed)
+    sites = np.stack(np.meshgrid(*[np.arange(q) for q in k], indexing="ij"), -1).reshape(-1, 3)
+    sites = sites[np.sort(rng.permutation(len(sites))[:n])]
+    s = water.water_box(2, rc=rc, ron=rc - 1.0, seed=seed, nmol=1, box=20.0)
+    o, h = s["pos"][0], s["pos"][1:3] - s["pos"][0]
+    first = (sites + 0.5) * (region / k) + rng.uniform(-0.1, 0.1, (n, 3)) + 0.5 * (edges - region)
+    turn = np.linalg.qr(rng.standard_normal((n, 3, 3)))[0]
+    pos = np.concatenate([first[:, None], first[:, None] + np.einsum("nij,hj->nhi", turn, h)], 1)
+    s.update(pos=pos.reshape(-1, 3), type=np.tile(s["type"], n), qscaled=np.tile(s["qscaled"], n),
+             mass=np.tile(s["mass"], n), mol=np.repeat(np.arange(n, dtype=np.int32), 3),
+             excl=(np.tile(s["excl"], (n, 1)) +
+                   np.repeat(3 * np.arange(n), 3)[:, None] * np.array([1, 1, 0])).astype(np.int32),
+             box=edges, origin=0.5 * edges, n=3 * n)
+    return s
+
+
+def _merged(s, size, modified):
+    """`size` neighbouring waters as one molecule, all its pairs excluded or (one
+    in three between different waters, where asked) modified."""
+    n = s["n"]
+    s["mol"] = (np.arange(n) // (3 * size)).astype(np.int32)
+    a, b = np.triu_indices(3 * size, 1)
+    kind = np.where(modified & (a // 3 != b // 3) & ((a + b) % 3 == 0), 1, 2)
+    base = np.arange(0, n, 3 * size)
+    e = np.stack([(base[:, None] + a).ravel(), (base[:, None] + b).ravel(),
+                  np.tile(kind, len(base))], -1)
+    s["excl"] = e[(e[:, 0] < n) & (e[:, 1] < n)].astype(np.int32)
+    s["lj"] = s["lj"] * np.array([1.0, 1.0, 0.5, 0.5])
+    s["coulomb_scaling"] = 0.8
+    return s
+
+
+def _unwrapped(s):
+    rng = np.random.default_rng(5)
+    s["pos"] = s["pos"] + np.repeat(rng.integers(-2, 3, (s["n"] // 3, 3)), 3, 0) * s["box"]
+    return s
+
+
+CASES = {
+    "one_water": lambda: _waters(1, (16.0, 16.0, 16.0)),
+    "three_waters": lambda: _waters(3, (17.0, 19.0, 16.5)),
+    "two_cutoffs": lambda: _waters(136, (16.0, 16.0, 16.0)),
+    "odd_edges_unwrapped": lambda: _unwrapped(_waters(509, (16.1, 22.3, 45.0))),
+    "dilute_tall_clusters": lambda: _waters(61, (27.0, 33.0, 46.0), rc=12.0),
+    "one_full_column": lambda: _waters(331, (60.0, 60.0, 100.0), (9.0, 9.0, 99.0)),
+    "long_columns": lambda: _waters(10007, (16.5, 16.5, 1110.0)),
+    "long_exclusion_lists": lambda: _merged(_waters(400, (20.0, 25.0, 24.0)), 4, False),
+    "modified_pairs": lambda: _merged(_waters(399, (20.0, 25.0, 24.0)), 3, True),
+    "flat": lambda: _waters(700, (60.0, 21.0, 16.0)),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_against_oracle(name):
+    s = CASES[name]()
+    n = s["n"]
+    topo = PeriodicTopology.from_dict(s)
+    f = NonbondedCutoffB200SystemForce(s["ron"], s["rc_lj"], s["rc_coul"], s["rc_alg"])
+    F = np.zeros_like(s["pos"])
+    E = ScalarStructure(virial=True, molecular_virial=True)
+    f.evaluate(topo, s["pos"], F, E)
+    pairs = f.last_pair_count()
+    F2, E2 = np.zeros_like(F), ScalarStructure()
+    f.evaluate(topo, s["pos"], F2, E2)  # the instance without virial, the counts cleared
+    f.close()
+    fo, eo, vo, mo = O.restate_eval(s, s["pos"], virial_mode=2)
+    assert np.array_equal(F, F2)
+    scale = max(np.sqrt((fo ** 2).sum()), 1e-30)
+    assert np.sqrt(((F - fo) ** 2).sum()) <= 1e-5 * scale
+    for e in (E, E2):
+        assert abs(e[0] - eo[0]) <= 1e-4 * n and abs(e[1] - eo[1]) <= 1e-4 * n
+    po = O.restate_count_pairs(s, s["pos"])
+    assert abs(pairs - po) <= 1 + 1e-6 * po
+    for got, want in ((E.virial_matrix(), vo), (E.molvirial_matrix(), mo)):
+        want = np.asarray(want).reshape(3, 3)
+        assert np.abs(got - want).max() <= 1e-5 * max(np.abs(want).max(), 1.0)
