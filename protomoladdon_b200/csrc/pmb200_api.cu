@@ -1334,7 +1334,8 @@ int launch_eval(pmb200_ctx *c, const double *d_pos, double *d_forces, double *d_
     return launch_eval_clusters(c, d_pos, d_forces, d_out, flags, accumulate, st,
                                 c->timing && cs == cudaStreamCaptureStatusNone);
   }
-  if (columns_apply(c, flags))
+  // (the FP64 column kernels serve evaluations without virial)
+  if (columns_apply(c, flags) || (c->col_ok && !mixed && !virial))
     return launch_eval_columns(c, d_pos, d_forces, d_out, flags, accumulate, st, f32, tail,
                                packed);
   // the cell build clears the accumulator on the way (still in L2 when the
@@ -2348,7 +2349,7 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
   // a Hessian-vector product asked for neither parameter derivative skips them
   const bool params = mode == DERIV_PARAMS || d_dq || d_dlj;
   const bool half = !params || c->ntypes <= kDerivRegTypes;
-  const bool col = false;
+  const bool col = half && c->col_ok;  // the column kernels serve the half shell's cases
   const int blocks = col ? c->col_clusters << c->col_lsplit
                          : (half ? g.ncell * kDerivSlots : (g.ncell + 3) / 4);
   if (params) {
