@@ -1193,7 +1193,8 @@ int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
   launch_k(k_col_sort, (unsigned)g.ncol, kColSortThreads, 0, st, true, n, g,
            (const int4 *)c->d_ipos, (const int *)c->d_ccount, (const int *)c->d_bucket,
            (const int *)c->d_type, (const int *)c->d_mol, (const unsigned char *)c->d_ljact,
-           (const double *)c->d_q, c->d_cspos, c->d_csmeta, c->d_csq, c->d_zs, c->d_cscratch,
+           (const double *)c->d_q, c->d_cspos, c->d_csmeta, c->d_csq, c->d_sidx, c->d_zs,
+           c->d_cscratch,
            c->d_cctl, fp64 ? (const double4 *)c->d_dpos : (const double4 *)nullptr,
            fp64 ? c->d_cspos64 : (double4 *)nullptr, d_w, d_w ? c->d_cw : (double4 *)nullptr);
   CK(cudaGetLastError());
@@ -1213,6 +1214,7 @@ ColArrays col_arrays(const pmb200_ctx *c) {
   a.ex_start = c->d_ex_start;
   a.ex = c->d_ex;
   a.icom = c->d_icom;
+  a.n = c->n;
   a.err = c->d_err;
   return a;
 }
@@ -1288,12 +1290,12 @@ int launch_eval_columns(pmb200_ctx *c, const double *d_pos, double *d_forces, do
     c->col_count_zero = true;  // (the kernel clears the counts)
   }
   const double scale = kFixInv / c->col_unit;
-  const int ns = virial ? ACC_MV : ACC_E, n3 = 3 * n;
+  const int ns = virial ? ACC_MV : ACC_E;
   const int lsplit = c->col_lsplit;
   if ((energy || virial) && !timed) {
     launch_k(mixed ? k_col_finalize_reduce<false> : k_col_finalize_reduce<true>,
-             (unsigned)std::max((n3 + 255) / 256, kRedBlocks), 256, 0, st, true, n,
-             (const unsigned long long *)c->d_facc, scale, accumulate, d_forces,
+             (unsigned)std::max((n + 255) / 256, kRedBlocks), 256, 0, st, true, n,
+             (const unsigned long long *)c->d_facc, (const int *)c->d_sidx, scale, accumulate, d_forces,
              (const int *)c->d_cctl, lsplit, (const double *)c->d_cpartial, c->d_red,
              c->d_redctr, d_out ? d_out : c->d_out, c->d_pairs, ns, f32, tail,
              (const int *)c->d_err);
@@ -1301,9 +1303,9 @@ int launch_eval_columns(pmb200_ctx *c, const double *d_pos, double *d_forces, do
     CK(cudaGetLastError());
     return PMB200_OK;
   }
-  launch_k(mixed ? k_col_finalize<false> : k_col_finalize<true>, (unsigned)((n3 + 255) / 256),
-           256, 0, st, !timed, n, (const unsigned long long *)c->d_facc, scale, accumulate,
-           d_forces, (double *)nullptr);
+  launch_k(mixed ? k_col_finalize<false> : k_col_finalize<true>, (unsigned)((n + 255) / 256),
+           256, 0, st, !timed, n, (const unsigned long long *)c->d_facc, (const int *)c->d_sidx,
+           scale, accumulate, d_forces, (double *)nullptr);
   if (timed) CK(cudaEventRecord(c->ev1, st));
   if (energy || virial) {
     k_col_reduce1<<<kRedBlocks, 256, 0, st>>>(c->d_cctl, lsplit, ColShare{0, 1, 1},
@@ -2323,8 +2325,8 @@ int pmb200_shard_finalize(pmb200_ctx *c, const long long *d_facc, double *d_forc
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   const unsigned long long *facc = reinterpret_cast<const unsigned long long *>(d_facc);
   if (c->n > 0 && c->col_ok)
-    k_col_finalize<false><<<(3 * c->n + 255) / 256, 256, 0, st>>>(
-        c->n, facc, kFixInv / c->col_unit, 1, d_forces, nullptr);
+    k_col_finalize<false><<<(c->n + 255) / 256, 256, 0, st>>>(
+        c->n, facc, c->d_sidx, kFixInv / c->col_unit, 1, d_forces, nullptr);
   else if (c->n > 0)
     k_finalize<<<(c->n + 255) / 256, 256, 0, st>>>(c->n, facc, c->d_sidx, kFixInv / c->g.unit, 1,
                                                   d_forces);
@@ -2379,8 +2381,8 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
     l.tpart = c->d_tpart;
     CK(col_launch_deriv64(c->cg, c->fc, col_arrays(c), l, mode, params, st));
     c->col_count_zero = true;  // (the kernel clears the counts)
-    launch_k(k_col_finalize<true>, (unsigned)((3 * n + 255) / 256), 256, 0, st, true, n,
-             (const unsigned long long *)c->d_facc, 1.0, 0,
+    launch_k(k_col_finalize<true>, (unsigned)((n + 255) / 256), 256, 0, st, true, n,
+             (const unsigned long long *)c->d_facc, (const int *)c->d_sidx, 1.0, 0,
              mode == DERIV_VJP ? d_hv : (double *)nullptr, params ? d_dq : (double *)nullptr);
     if (params)
       k_reduce_columns<<<(unsigned)nt4, 1024, 0, st>>>(blocks, (int)nt4, c->d_tpart, d_dlj);
@@ -2779,8 +2781,8 @@ int pmb200_eval_cells(pmb200_ctx *c, const double *pos, double *forces, double *
     }
     rc = launch_col_pair(c, flags, st, true, share, c->d_facc);
     if (rc) return rc;
-    k_col_finalize<false><<<(3 * c->n + 255) / 256, 256, 0, st>>>(
-        c->n, c->d_facc, kFixInv / c->col_unit, 0, c->d_hfrc, nullptr);
+    k_col_finalize<false><<<(c->n + 255) / 256, 256, 0, st>>>(
+        c->n, c->d_facc, c->d_sidx, kFixInv / c->col_unit, 0, c->d_hfrc, nullptr);
     if (energy || anyvir) {
       const int ns = anyvir ? ACC_MV : ACC_E;
       k_col_reduce1<<<kRedBlocks, 256, 0, st>>>(c->d_cctl, c->col_lsplit, share, c->d_cpartial,
@@ -3653,6 +3655,7 @@ ColBatchLaunch batch_col_launch(const pmb200_batch *b, bool energy, bool virial,
   a.ex_start = b->d_ex_start;
   a.ex = b->d_ex;
   a.facc = b->d_facc;
+  a.n = b->N;
   a.err = b->d_err;
   ColBatchLaunch l{};
   l.form = b->form;
@@ -3693,7 +3696,8 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
                                                        b->d_facc, b->d_err);
     k_col_sort_batch<<<b->ncol, kColSortThreads, 0, st>>>(
         b->d_col, b->d_col_sys, b->d_ipos, b->d_ccount, b->d_bucket, b->d_type, b->d_mol,
-        b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_zs, b->d_scratch, b->d_ctl);
+        b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_sidx, b->d_zs, b->d_scratch,
+        b->d_ctl);
     BCK(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
     ColArrays a{};
     ColBatchLaunch l = batch_col_launch(b, energy, virial, a);
@@ -3704,8 +3708,8 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
     BCK(col_launch_batch(a, l, st, nullptr));
     b->col_dirty = false;  // (the kernel clears the counts)
     if (timed) BCK(cudaEventRecord(b->ev1, st));
-    k_col_finalize_batch<<<(3 * N + 255) / 256, 256, 0, st>>>(N, b->d_facc, b->d_atom_sys,
-                                                              b->d_col, accumulate, d_forces);
+    k_col_finalize_batch<<<(N + 255) / 256, 256, 0, st>>>(N, b->d_facc, b->d_sidx, b->d_atom_sys,
+                                                          b->d_col, accumulate, d_forces);
     if ((energy || virial) && d_out)
       k_reduce_batch<<<b->nsys, 128, 0, st>>>(b->d_rows_start, b->d_rows, b->d_partial, d_out,
                                                b->d_pairs, virial ? ACC_MV : ACC_E);

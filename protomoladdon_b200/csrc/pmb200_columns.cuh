@@ -20,11 +20,15 @@
 //   ipos[n]     int4  {x, y, z fractions, charge (FP32 bits)}, caller order
 //   bucket[ncol][cap] int  atoms of a column in arrival order
 //   spos[S]     int4  ipos in column / height order
-//   smeta[S]    int4  {type | LJ-active << 16, molecule, atom (-1: pad), 0}
+//   smeta[S]    int4  {type | LJ-active << 16, molecule, atom (-1: pad), rank}; rank:
+//                     the atom's place in column / height order without the pads
+//   sidx[n]     int   the atom of each rank
 //   sq[S]       double charge (FP64; energies)
 //   dpos[n], spos64[S] double4 {wrapped position (A), charge} (FP64 kernels)
 //   zs[ncol][nsz + 1] int  first slot of a column at or above a slab's bottom
-//   facc[n][3]  int64 fixed-point forces, caller order
+//   facc[3][n]  int64 fixed-point forces, by rank (a block's atoms lie close
+//               together: in the caller's order its atomics took four times the
+//               memory wavefronts)
 #pragma once
 #include "pmb200_kernels.cuh"
 
@@ -129,7 +133,7 @@ static __global__ void k_col_index(int n, const double *__restrict__ pos, ColGri
   ipos[i] = make_int4((int)u[0], (int)u[1], (int)u[2], __float_as_int((float)q[i] * g.qscale));
 }
 
-// One column's sort by one block: base is its first slot.  Order: slab, height,
+// One column's sort by one block: base is its first slot, rank0 its first rank.  Order: slab, height,
 // atom index (the layout, and every sum over it, is the same on every run).
 // A counting sort by slab in shared memory, then ranks among the two or three
 // atoms of a slab; the slabs' first slots come with it.  (Ranks counted against
@@ -144,11 +148,11 @@ struct ColSortSmem {
   int warp[8], n;
 };
 __device__ __forceinline__ void col_sort_column(
-    const ColGrid &g, int col, int cnt, int base, int i0, int n, const int4 *__restrict__ ipos,
+    const ColGrid &g, int col, int cnt, int base, int rank0, int i0, int n, const int4 *__restrict__ ipos,
     const int *__restrict__ bucket, const int *__restrict__ type, const int *__restrict__ mol,
     const unsigned char *__restrict__ ljact, const double *__restrict__ q,
     int4 *__restrict__ spos, int4 *__restrict__ smeta, double *__restrict__ sq,
-    int *__restrict__ zs, int *scratch, ColSortSmem &sm,
+    int *__restrict__ sidx, int *__restrict__ zs, int *scratch, ColSortSmem &sm,
     const double4 *__restrict__ dpos = nullptr, double4 *__restrict__ spos64 = nullptr,
     const double *__restrict__ w = nullptr, double4 *__restrict__ sw = nullptr) {
   const int T = blockDim.x, t = threadIdx.x, lane = t & 31, wp = t >> 5;
@@ -157,7 +161,8 @@ __device__ __forceinline__ void col_sort_column(
     const int ty = type[i], mo = mol[i];
     const double qi = q[i];
     spos[base + rank] = p;
-    smeta[base + rank] = make_int4(ty | ((int)ljact[ty] << 16), mo, i, 0);
+    smeta[base + rank] = make_int4(ty | ((int)ljact[ty] << 16), mo, i, rank0 + rank);
+    sidx[rank0 + rank] = i;
     sq[base + rank] = qi;
     if (spos64) spos64[base + rank] = dpos[i];
     if (sw)
@@ -249,35 +254,54 @@ __device__ __forceinline__ void col_sort_column(
   }
 }
 
+// The clusters and atoms of the columns before `col` (each block sums them
+// itself: a few thousand counts at most on the sizes a GPU holds, and no scan
+// launch).
+__device__ __forceinline__ void col_before(const int *__restrict__ count, int col, int &clusters,
+                                           int &atoms, ColSortSmem &sm) {
+  const int t = threadIdx.x;
+  int s = 0, a = 0;
+  for (int c = t; c < col; c += kColSortThreads) {
+    const int v = count[c];
+    a += v;
+    s += (v + kColI - 1) / kColI;
+  }
+  s = __reduce_add_sync(0xffffffffu, s);
+  a = __reduce_add_sync(0xffffffffu, a);
+  if ((t & 31) == 0) {
+    sm.warp[t >> 5] = s;
+    sm.list[t >> 5] = a;
+  }
+  __syncthreads();
+  clusters = atoms = 0;
+#pragma unroll
+  for (int w = 0; w < kColSortThreads / 32; w++) {
+    clusters += sm.warp[w];
+    atoms += sm.list[w];
+  }
+}
+
 // One block per column.  ctl[0]: the number of clusters.
 static __global__ void __launch_bounds__(kColSortThreads)
 k_col_sort(int n, ColGrid g, const int4 *__restrict__ ipos, const int *__restrict__ count,
            const int *__restrict__ bucket, const int *__restrict__ type,
            const int *__restrict__ mol, const unsigned char *__restrict__ ljact,
            const double *__restrict__ q, int4 *__restrict__ spos, int4 *__restrict__ smeta,
-           double *__restrict__ sq, int *__restrict__ zs, int *__restrict__ scratch,
-           int *__restrict__ ctl, const double4 *__restrict__ dpos,
+           double *__restrict__ sq, int *__restrict__ sidx, int *__restrict__ zs,
+           int *__restrict__ scratch, int *__restrict__ ctl, const double4 *__restrict__ dpos,
            double4 *__restrict__ spos64, const double *__restrict__ w,
            double4 *__restrict__ sw) {
   pdl_trigger();
   pdl_wait();
   __shared__ ColSortSmem sm;
   const int col = blockIdx.x, t = threadIdx.x;
-  // the slots of the columns before this one (each block sums them itself:
-  // a few thousand counts at most on the sizes a GPU holds, and no scan launch)
-  int s = 0;
-  for (int c = t; c < col; c += kColSortThreads) s += (count[c] + kColI - 1) / kColI;
-  s = __reduce_add_sync(0xffffffffu, s);
-  if ((t & 31) == 0) sm.warp[t >> 5] = s;
-  __syncthreads();
-  int before = 0;
-#pragma unroll
-  for (int w = 0; w < kColSortThreads / 32; w++) before += sm.warp[w];
+  int before, atoms;
+  col_before(count, col, before, atoms, sm);
   const int cnt = count[col];
   if (col == g.ncol - 1 && t == 0) ctl[0] = before + (cnt + kColI - 1) / kColI;
   __syncthreads();
-  col_sort_column(g, col, cnt, before * kColI, 0, n, ipos, bucket + (size_t)col * g.cap, type,
-                  mol, ljact, q, spos, smeta, sq, zs + (size_t)col * (g.nsz + 1), scratch, sm,
+  col_sort_column(g, col, cnt, before * kColI, atoms, 0, n, ipos, bucket + (size_t)col * g.cap,
+                  type, mol, ljact, q, spos, smeta, sq, sidx, zs + (size_t)col * (g.nsz + 1), scratch, sm,
                   dpos, spos64, w, sw);
 }
 
@@ -582,7 +606,8 @@ struct ColArrays {  // per system (single) or batch-wide
   const int *ex_start;
   const int2 *ex;
   const int4 *icom;
-  unsigned long long *facc;  // [n][3]
+  unsigned long long *facc;  // [3][n]
+  int n;
   int *err;
 };
 
@@ -645,7 +670,7 @@ constexpr float kColForceLim = 1.0e9f;          // summed force component (unit 
 // bytes), {meta, force offset} (8), for the exact energies the FP64 charge (8), for
 // the molecular virial the molecule's centre (16) -- then the cluster's molecules
 // and the candidate runs.  meta: 16 type | pair mask << 16 | modified mask << 24;
-// force offset: 24 atom.
+// force offset: 8 rank.
 template <bool kExactE, bool kMolVir>
 struct ColLayout {
   static constexpr unsigned pos = 0, mg = 16 * kColCap, qd = mg + 8 * kColCap,
@@ -880,8 +905,8 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
       unsigned long long *f = reinterpret_cast<unsigned long long *>(
           reinterpret_cast<char *>(A.facc) + off);
       atomicAdd(f, (unsigned long long)__float2ll_rn(jx * kColFix));
-      atomicAdd(f + 1, (unsigned long long)__float2ll_rn(jy * kColFix));
-      atomicAdd(f + 2, (unsigned long long)__float2ll_rn(jz * kColFix));
+      atomicAdd(f + A.n, (unsigned long long)__float2ll_rn(jy * kColFix));
+      atomicAdd(f + 2 * (size_t)A.n, (unsigned long long)__float2ll_rn(jz * kColFix));
     }
   };
   auto copy_entry = [&](int from, int to) {
@@ -957,7 +982,7 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
           sts4(sb + Lay::pos + 16 * e, p);
           if (kExactE) sts1d(sb + Lay::qd + 8 * e, qd);
           sts2(sb + Lay::mg + 8 * e, ((m.x & 0xfff) << 4) | (pmask.x << 16) | (pmask.y << 24),
-               (int)(24u * (unsigned)m.z));
+               (int)(8u * (unsigned)m.w));
           if (kMolVir) sts4(sb + Lay::com + 16 * e, A.icom[m.y]);
         }
         nl += __popc(kf);
@@ -974,7 +999,7 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
   }
   if (active && js < 3) {
     const long long v = js == 0 ? fx : (js == 1 ? fy : fz);
-    if (v) atomicAdd(&A.facc[3 * (size_t)mi.z + js], (unsigned long long)v);
+    if (v) atomicAdd(&A.facc[(size_t)js * A.n + mi.w], (unsigned long long)v);
   }
   if (kEnergy || kVirial) {
     double v[ACC_MV];
@@ -1045,30 +1070,38 @@ k_col_pair(const ColGrid g, const MixedConsts mc, int ntypes, const float4 *__re
       partial + (size_t)blockIdx.x * kNacc);
 }
 
-// Component q of atom i's force from the fixed-point sums: [n][3] (mixed; scale
-// 2^-32 / unit) or the FP64 kernels' two words [n][8] (unscaled; q = 3: dq).
+// Component q of the force on the atom of rank r from the fixed-point sums: [3][n]
+// (mixed; scale 2^-32 / unit) or the FP64 kernels' two words [8][n] (unscaled; q =
+// 3: dq).
 template <bool k64>
-__device__ __forceinline__ double col_force(const unsigned long long *__restrict__ facc, int i,
-                                            int q, double scale) {
-  if (!k64) return (double)(long long)facc[3 * (size_t)i + q] * scale;
-  const double hi = (double)(long long)facc[8 * (size_t)i + q];
-  const double lo = (double)(long long)facc[8 * (size_t)i + 4 + q];
+__device__ __forceinline__ double col_force(const unsigned long long *__restrict__ facc, size_t n,
+                                            int r, int q, double scale) {
+  if (!k64) return (double)(long long)facc[q * n + r] * scale;
+  const double hi = (double)(long long)facc[q * n + r];
+  const double lo = (double)(long long)facc[(4 + q) * n + r];
   return (hi + lo * (1.0 / kFix2Lo)) * (1.0 / kFix2Hi);
 }
 
-// Forces (or H w), accumulated or overwritten; dq (FP64 kernels, or null).
+// Forces (or H w) in the caller's order, accumulated or overwritten; dq (FP64
+// kernels, or null).
 template <bool k64>
 __global__ void __launch_bounds__(256)
-k_col_finalize(int n, const unsigned long long *__restrict__ facc, double scale, int accumulate,
-               double *__restrict__ forces, double *__restrict__ dq) {
+k_col_finalize(int n, const unsigned long long *__restrict__ facc, const int *__restrict__ sidx,
+               double scale, int accumulate, double *__restrict__ forces,
+               double *__restrict__ dq) {
   pdl_wait();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < 3 * n && forces) {
-    const int i = k / 3;
-    const double v = col_force<k64>(facc, i, k - 3 * i, scale);
-    forces[k] = accumulate ? forces[k] + v : v;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int o = sidx[r];
+  if (forces) {
+    double *f = forces + 3 * (size_t)o;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const double v = col_force<k64>(facc, n, r, q, scale);
+      f[q] = accumulate ? f[q] + v : v;
+    }
   }
-  if (k64 && dq && k < n) dq[k] = col_force<k64>(facc, k, 3, scale);
+  if (k64 && dq) dq[o] = col_force<k64>(facc, n, r, 3, scale);
 }
 
 // k_reduce1 over the rows of a share's clusters.
@@ -1084,14 +1117,14 @@ static __global__ void k_col_reduce1(const int *__restrict__ ctl, int lsplit, Co
 }
 
 // k_col_finalize, k_col_reduce1 and k_reduce2 in one launch of
-// max(ceil(3 n / 256), kRedBlocks) blocks (see k_finalize_reduce: the same sums
+// max(ceil(n / 256), kRedBlocks) blocks (see k_finalize_reduce: the same sums
 // in the same order as the separate kernels).  f32: the forces go there in FP32
 // instead.  tail (or null): receives the 20 results and the error flag.
 template <bool k64>
 __global__ void __launch_bounds__(256)
-k_col_finalize_reduce(int n, const unsigned long long *__restrict__ facc, double scale,
-                      int accumulate, double *__restrict__ forces, const int *__restrict__ ctl,
-                      int lsplit, const double *__restrict__ partial, double *red,
+k_col_finalize_reduce(int n, const unsigned long long *__restrict__ facc,
+                      const int *__restrict__ sidx, double scale, int accumulate,
+                      double *__restrict__ forces, const int *__restrict__ ctl, int lsplit, const double *__restrict__ partial, double *red,
                       unsigned *__restrict__ arrivals, double *__restrict__ out,
                       double *__restrict__ pairs_out, int ns, float *__restrict__ f32,
                       double *tail, const int *err) {
@@ -1099,12 +1132,15 @@ k_col_finalize_reduce(int n, const unsigned long long *__restrict__ facc, double
   __shared__ double sh[8][ACC_MV];
   __shared__ double col[ACC_MV];
   __shared__ unsigned s_arrived;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < 3 * n) {
-    const int i = k / 3;
-    const double v = col_force<k64>(facc, i, k - 3 * i, scale);
-    if (f32) f32[k] = (float)v;
-    else forces[k] = accumulate ? forces[k] + v : v;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < n) {
+    const size_t o = 3 * (size_t)sidx[r];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const double v = col_force<k64>(facc, n, r, q, scale);
+      if (f32) f32[o + q] = (float)v;
+      else forces[o + q] = accumulate ? forces[o + q] + v : v;
+    }
   }
   if (blockIdx.x >= kRedBlocks) return;  // uniform per block
   reduce1_block(blockIdx.x, col_rows(ctl, lsplit, ColShare{0, 1, 1}), partial, red, ns, sh);
@@ -1124,7 +1160,7 @@ k_col_finalize_reduce(int n, const unsigned long long *__restrict__ facc, double
 
 // ---------------------------------------------------------------------------
 // Batches of systems: the same kernels over concatenated arrays.  Atom indices
-// (ipos, smeta, facc, the exclusion lists) are batch-wide; slots, columns and
+// and ranks (ipos, smeta, facc, the exclusion lists) are batch-wide; slots, columns and
 // clusters count from each system's first.
 // ---------------------------------------------------------------------------
 struct ColBatchSys {
@@ -1163,28 +1199,20 @@ k_col_sort_batch(const ColBatchSys *__restrict__ sys, const int *__restrict__ co
                  const int *__restrict__ bucket, const int *__restrict__ type,
                  const int *__restrict__ mol, const unsigned char *__restrict__ ljact,
                  const double *__restrict__ q, int4 *__restrict__ spos,
-                 int4 *__restrict__ smeta, double *__restrict__ sq, int *__restrict__ zs,
-                 int *__restrict__ scratch, int *__restrict__ ctl) {
+                 int4 *__restrict__ smeta, double *__restrict__ sq, int *__restrict__ sidx,
+                 int *__restrict__ zs, int *__restrict__ scratch, int *__restrict__ ctl) {
   __shared__ ColSortSmem sm;
   const int s = col_sys[blockIdx.x], t = threadIdx.x;
   const ColBatchSys &b = sys[s];
   const int col = (int)blockIdx.x - b.col0;
-  int before = 0;
-  {
-    int v = 0;
-    for (int c = t; c < col; c += kColSortThreads) v += (count[b.col0 + c] + kColI - 1) / kColI;
-    v = __reduce_add_sync(0xffffffffu, v);
-    if ((t & 31) == 0) sm.warp[t >> 5] = v;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < kColSortThreads / 32; w++) before += sm.warp[w];
-  }
+  int before, atoms;
+  col_before(count + b.col0, col, before, atoms, sm);
   const int cnt = count[blockIdx.x];
   if (col == b.g.ncol - 1 && t == 0) ctl[s] = before + (cnt + kColI - 1) / kColI;
   __syncthreads();
-  col_sort_column(b.g, col, cnt, before * kColI, b.atom0, b.natoms, ipos,
+  col_sort_column(b.g, col, cnt, before * kColI, b.atom0 + atoms, b.atom0, b.natoms, ipos,
                   bucket + b.bucket0 + (size_t)col * b.g.cap, type, mol, ljact + b.act0, q,
-                  spos + b.slot0, smeta + b.slot0, sq + b.slot0,
+                  spos + b.slot0, smeta + b.slot0, sq + b.slot0, sidx,
                   zs + b.zs0 + (size_t)col * (b.g.nsz + 1), scratch + b.slot0, sm);
 }
 
@@ -1252,12 +1280,19 @@ k_col_pair_batch(const ColBatchSys *__restrict__ sys, const int4 *__restrict__ t
 
 static __global__ void __launch_bounds__(256)
 k_col_finalize_batch(int N, const unsigned long long *__restrict__ facc,
-                     const int *__restrict__ atom_sys, const ColBatchSys *__restrict__ sys,
-                     int accumulate, double *__restrict__ forces) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= 3 * N) return;
-  const double v = (double)(long long)facc[k] * sys[atom_sys[k / 3]].fscale;
-  forces[k] = accumulate ? forces[k] + v : v;
+                     const int *__restrict__ sidx, const int *__restrict__ atom_sys,
+                     const ColBatchSys *__restrict__ sys, int accumulate,
+                     double *__restrict__ forces) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= N) return;
+  const int o = sidx[r];
+  const double scale = sys[atom_sys[o]].fscale;
+  double *f = forces + 3 * (size_t)o;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const double v = col_force<false>(facc, N, r, q, scale);
+    f[q] = accumulate ? f[q] + v : v;
+  }
 }
 
 }  // namespace pmb200

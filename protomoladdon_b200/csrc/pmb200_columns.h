@@ -48,7 +48,7 @@ struct Col64Launch {
   bool full;               // cutoff form: both switches end at the cutoff, no modified pairs
   bool energy, pdl;
   const double4 *lj64;     // {A, B, A14, B14}
-  unsigned long long *acc; // [n][8]
+  unsigned long long *acc; // [8][n]
   const int *ctl;
   int *count;
   int lsplit, clusters;

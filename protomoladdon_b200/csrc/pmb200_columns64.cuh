@@ -5,20 +5,22 @@
 // margin); positions, pair arithmetic and sums are FP64.
 //
 // Sums: each lane's i terms in registers (added over the lane groups in a fixed
-// order), j terms travelling with the walk; both reach acc[n][8] (caller order,
-// words {hi x, hi y, hi z, hi q, lo x, lo y, lo z, lo q}) as the exact two-word
+// order), j terms travelling with the walk; both reach acc[8][n] (by rank,
+// rows hi x, hi y, hi z, hi q, lo x, lo y, lo z, lo q) as the exact two-word
 // fixed point of fix2_add, so the results are bitwise reproducible.
 #pragma once
 #include "pmb200_columns.cuh"
 
 namespace pmb200 {
 
-// Staged entries: {x, y, z, q} FP64 (32 bytes), {meta, atom} (8), for products the
-// direction (32); meta: type | pair mask << 16 | modified mask << 24.
+// Staged entries: {x, y} and {z, q} FP64 in arrays of their own (16 bytes an entry:
+// no bank conflicts), {meta, rank} (8), for products the direction {x, y}, {z, 0};
+// meta: type | pair mask << 16 | modified mask << 24.
 template <bool kW>
 struct ColLayout64 {
-  static constexpr unsigned pos = 0, mg = 32 * kColCap, w = mg + 8 * kColCap,
-                            mol = w + (kW ? 32 * kColCap : 0), runs = mol + 32,
+  static constexpr unsigned half = 16 * kColCap;  // {x, y} to {z, q}
+  static constexpr unsigned pos = 0, mg = 2 * half, w = mg + 8 * kColCap,
+                            mol = w + (kW ? 2 * half : 0), runs = mol + 32,
                             bytes = (runs + 256 + 511) / 512 * 512;
 };
 
@@ -31,9 +33,9 @@ __device__ __forceinline__ void sts2d(unsigned a, double x, double y) {
   asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(x), "d"(y) : "memory");
 }
 
-// v into word q (0..3) of atom j's accumulator (fix2_add's split)
-__device__ __forceinline__ void fix2_add_atom(unsigned long long *__restrict__ acc, int j, int q,
-                                              double v, int *__restrict__ err) {
+// v into word q (0..3) of the atom of rank r (fix2_add's split)
+__device__ __forceinline__ void fix2_add_rank(unsigned long long *__restrict__ acc, size_t n, int r,
+                                              int q, double v, int *__restrict__ err) {
   if (v == 0.0) return;
   if (!(fabs(v) < kFix2Max)) {
     atomicOr(err, 2);
@@ -43,11 +45,12 @@ __device__ __forceinline__ void fix2_add_atom(unsigned long long *__restrict__ a
   const double h = rint(s);
   const long long hi = (long long)h;
   const long long lo = __double2ll_rn((s - h) * kFix2Lo);
-  if (hi) atomicAdd(&acc[8 * (size_t)j + q], (unsigned long long)hi);
-  if (lo) atomicAdd(&acc[8 * (size_t)j + 4 + q], (unsigned long long)lo);
+  if (hi) atomicAdd(&acc[q * n + r], (unsigned long long)hi);
+  if (lo) atomicAdd(&acc[(4 + q) * n + r], (unsigned long long)lo);
 }
+
 // The walk common to both kernels.  Pair: a functor with
-//   pair(front, a32, a8)   this lane's atom against the entry there
+//   pair(front, a16, a8)   this lane's atom against the entry there
 //   start()                zero the j terms
 //   shift(to)              the j terms moved to the lane `to` away
 //   finish(a8)             the j terms (whole) added to the entry's atom
@@ -61,28 +64,28 @@ struct ColWalk64 {
   template <class Tag>
   __device__ __forceinline__ void block(Tag tag, int e0) {
     const unsigned e = (unsigned)(e0 + (threadIdx.x & 31));
-    unsigned a32 = sb + Lay::pos + 32 * e, a8 = sb + Lay::mg + 8 * e;
+    unsigned a16 = sb + Lay::pos + 16 * e, a8 = sb + Lay::mg + 8 * e;
     pair.start();
 #pragma unroll 1
     for (int h = 0; h < 4; h++) {
 #pragma unroll
       for (int k = 0; k < 2; k++) {
         const unsigned to = k == 0 ? 1u : (h & 1 ? 7u : 3u);
-        pair(tag, a32, a8);
+        pair(tag, a16, a8);
         pair.shift((int)to);
-        a32 ^= to << 5;
+        a16 ^= to << 4;
         a8 ^= to << 3;
       }
     }
     pair.finish(a8);
   }
   __device__ __forceinline__ void copy(int from, int to) {
-    for (unsigned k = 0; k < 32; k += 16) {
-      const double2 d = lds2d(sb + Lay::pos + 32 * from + k);
-      sts2d(sb + Lay::pos + 32 * to + k, d.x, d.y);
+    for (unsigned h = 0; h <= Lay::half; h += Lay::half) {
+      const double2 d = lds2d(sb + Lay::pos + 16 * from + h);
+      sts2d(sb + Lay::pos + 16 * to + h, d.x, d.y);
       if (kW) {
-        const double2 v = lds2d(sb + Lay::w + 32 * from + k);
-        sts2d(sb + Lay::w + 32 * to + k, v.x, v.y);
+        const double2 v = lds2d(sb + Lay::w + 16 * from + h);
+        sts2d(sb + Lay::w + 16 * to + h, v.x, v.y);
       }
     }
     const int2 m = lds2(sb + Lay::mg + 8 * from);
@@ -104,9 +107,9 @@ struct ColWalk64 {
       fn = (nl + kColBlk - 1) & ~(kColBlk - 1);
       if (nl + lane < fn) {
         const int e = nl + lane;
-        for (unsigned k = 0; k < 32; k += 16) {
-          sts2d(sb + Lay::pos + 32 * e + k, 0.0, 0.0);
-          if (kW) sts2d(sb + Lay::w + 32 * e + k, 0.0, 0.0);
+        for (unsigned h = 0; h <= Lay::half; h += Lay::half) {
+          sts2d(sb + Lay::pos + 16 * e + h, 0.0, 0.0);
+          if (kW) sts2d(sb + Lay::w + 16 * e + h, 0.0, 0.0);
         }
         sts2(sb + Lay::mg + 8 * e, 0, 0);
       }
@@ -208,13 +211,13 @@ __device__ __forceinline__ void col_search64(const ColGrid &g, const ColArrays &
             s = make_double3(col_image((unsigned)p.x, a.box.xc, g.edge[0]),
                              col_image((unsigned)p.y, a.box.yc, g.edge[1]),
                              col_image((unsigned)p.z, a.box.zc, g.edge[2]));
-          sts2d(sb + Lay::pos + 32 * e, x.p.x + s.x, x.p.y + s.y);
-          sts2d(sb + Lay::pos + 32 * e + 16, x.p.z + s.z, x.p.w);
+          sts2d(sb + Lay::pos + 16 * e, x.p.x + s.x, x.p.y + s.y);
+          sts2d(sb + Lay::pos + 16 * e + Lay::half, x.p.z + s.z, x.p.w);
           if (kW) {
-            sts2d(sb + Lay::w + 32 * e, x.w.x, x.w.y);
-            sts2d(sb + Lay::w + 32 * e + 16, x.w.z, 0.0);
+            sts2d(sb + Lay::w + 16 * e, x.w.x, x.w.y);
+            sts2d(sb + Lay::w + 16 * e + Lay::half, x.w.z, 0.0);
           }
-          sts2(sb + Lay::mg + 8 * e, (m.x & 0xfff) | (pmask.x << 16) | (pmask.y << 24), m.z);
+          sts2(sb + Lay::mg + 8 * e, (m.x & 0xfff) | (pmask.x << 16) | (pmask.y << 24), m.w);
         }
         walk.nl += __popc(kf);
         walk.nn += __popc(kb);
@@ -257,9 +260,9 @@ struct ColPair64 {
 
   __device__ __forceinline__ void start() { jx = jy = jz = 0.0; }
   template <class Tag>
-  __device__ __forceinline__ void operator()(Tag, unsigned a32, unsigned a8) {
+  __device__ __forceinline__ void operator()(Tag, unsigned a16, unsigned a8) {
     constexpr bool kLj = Tag::value;
-    const double2 d0 = lds2d(a32), d1 = lds2d(a32 + 16);
+    const double2 d0 = lds2d(a16), d1 = lds2d(a16 + ColLayout64<false>::half);
     const int mj = lds1(a8);
     double d[3];
     double r2 = col_diff64(g, a, d0.x, d0.y, d1.x, d);
@@ -327,10 +330,10 @@ struct ColPair64 {
     jz = __shfl_xor_sync(0xffffffffu, jz, to);
   }
   __device__ __forceinline__ void finish(unsigned a8) {
-    const int j = lds1(a8 + 4);
-    fix2_add_atom(acc, j, 0, jx, A.err);
-    fix2_add_atom(acc, j, 1, jy, A.err);
-    fix2_add_atom(acc, j, 2, jz, A.err);
+    const int r = lds1(a8 + 4);
+    fix2_add_rank(acc, A.n, r, 0, jx, A.err);
+    fix2_add_rank(acc, A.n, r, 1, jy, A.err);
+    fix2_add_rank(acc, A.n, r, 2, jz, A.err);
   }
 };
 
@@ -377,7 +380,7 @@ k_col_pair64(const ColGrid g, const Fp64Consts mc, int ntypes, const double4 *__
   }
   const int js = lane / kColI;
   if (a.m.z >= 0 && js < 3)
-    fix2_add_atom(acc, a.m.z, js, js == 0 ? pair.fx : (js == 1 ? pair.fy : pair.fz), A.err);
+    fix2_add_rank(acc, A.n, a.m.w, js, js == 0 ? pair.fx : (js == 1 ? pair.fy : pair.fz), A.err);
   if (kEnergy) {
     double v[ACC_MV];
 #pragma unroll
@@ -412,10 +415,10 @@ struct ColDeriv64 {
 
   __device__ __forceinline__ void start() { jx = jy = jz = jq = 0.0; }
   template <class Tag>
-  __device__ __forceinline__ void operator()(Tag, unsigned a32, unsigned a8) {
+  __device__ __forceinline__ void operator()(Tag, unsigned a16, unsigned a8) {
     constexpr bool kLj = Tag::value;
     using Lay = ColLayout64<kVjp>;
-    const double2 d0 = lds2d(a32), d1 = lds2d(a32 + 16);
+    const double2 d0 = lds2d(a16), d1 = lds2d(a16 + Lay::half);
     const int mj = lds1(a8);
     double d[3];
     double s = col_diff64(g, a, d0.x, d0.y, d1.x, d);
@@ -438,7 +441,8 @@ struct ColDeriv64 {
     }
     double T = 0.0;
     if (kVjp) {
-      const double2 w0 = lds2d(a32 + (Lay::w - Lay::pos)), w1 = lds2d(a32 + (Lay::w - Lay::pos) + 16);
+      const double2 w0 = lds2d(a16 + (Lay::w - Lay::pos)),
+                    w1 = lds2d(a16 + (Lay::w - Lay::pos) + Lay::half);
       const double e0 = wx - w0.x, e1 = wy - w0.y, e2 = wz - w1.x;  // w_i - w_j
       const double dd = fma(d[0], e0, fma(d[1], e1, d[2] * e2));
       const double p = 2.0 * Us, q = 4.0 * Uss * dd;
@@ -488,13 +492,13 @@ struct ColDeriv64 {
     if (kParams) jq = __shfl_xor_sync(0xffffffffu, jq, to);
   }
   __device__ __forceinline__ void finish(unsigned a8) {
-    const int j = lds1(a8 + 4);
+    const int r = lds1(a8 + 4);
     if (kVjp) {
-      fix2_add_atom(acc, j, 0, jx, A.err);
-      fix2_add_atom(acc, j, 1, jy, A.err);
-      fix2_add_atom(acc, j, 2, jz, A.err);
+      fix2_add_rank(acc, A.n, r, 0, jx, A.err);
+      fix2_add_rank(acc, A.n, r, 1, jy, A.err);
+      fix2_add_rank(acc, A.n, r, 2, jz, A.err);
     }
-    if (kParams) fix2_add_atom(acc, j, 3, jq, A.err);
+    if (kParams) fix2_add_rank(acc, A.n, r, 3, jq, A.err);
   }
 };
 
@@ -552,8 +556,9 @@ k_col_deriv64(const ColGrid g, const Fp64Consts mc, int ntypes,
     const int js = lane / kColI;
     if (a.m.z >= 0) {
       if (kVjp && js < 3)
-        fix2_add_atom(acc, a.m.z, js, js == 0 ? pair.hx : (js == 1 ? pair.hy : pair.hz), A.err);
-      if (kParams && js == 3) fix2_add_atom(acc, a.m.z, 3, pair.gq, A.err);
+        fix2_add_rank(acc, A.n, a.m.w, js, js == 0 ? pair.hx : (js == 1 ? pair.hy : pair.hz),
+                      A.err);
+      if (kParams && js == 3) fix2_add_rank(acc, A.n, a.m.w, 3, pair.gq, A.err);
     }
     if (kParams) {
       // the lanes' register sums to both orders of the types, lane by lane (a
