@@ -43,10 +43,17 @@ __device__ __forceinline__ void fix2_add_rank(unsigned long long *__restrict__ a
   }
   const double s = v * kFix2Hi;
   const double h = rint(s);
-  const long long hi = (long long)h;
-  const long long lo = __double2ll_rn((s - h) * kFix2Lo);
-  if (hi) atomicAdd(&acc[q * n + r], (unsigned long long)hi);
-  if (lo) atomicAdd(&acc[(4 + q) * n + r], (unsigned long long)lo);
+  atomicAdd(&acc[q * n + r], (unsigned long long)(long long)h);
+  atomicAdd(&acc[(4 + q) * n + r], (unsigned long long)__double2ll_rn((s - h) * kFix2Lo));
+}
+
+// 1/sqrt(x) from the FP32 approximation y and one Halley step, y (1 + e/2 + 3 e^2/8)
+// with e = 1 - x y^2: e is about 2e-7, what is left out e^3 < 1e-20, so only the
+// step's roundings remain (about one unit in the last place).  x in FP32's range.
+__device__ __forceinline__ double col_rsqrt64(double x) {
+  const double y = (double)col_rsqrt((float)x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // The walk common to both kernels.  Pair: a functor with
@@ -274,7 +281,7 @@ struct ColPair64 {
       r2 = ok ? r2 : 1.0;
       double qj = ok ? d1.y : 0.0;
       if (!kFull) qj *= kind ? mc.csf : 1.0;
-      const double ir = rsqrt(r2), is = ir * ir;
+      const double ir = col_rsqrt64(r2), is = ir * ir;
       f = a.p.w * qj * fma(is, ir, -2.0 * mc.c05_3);
       double e = fma(mc.c05_3, r2, ir - mc.c15_1);
       if (!kFull) {
@@ -429,11 +436,11 @@ struct ColDeriv64 {
     double Us, Uss;
     DerivTerms u;
     if (kLj) {
-      u = deriv_terms(mc, lj, ti + tj, kind, s, d1.y);
+      u = deriv_terms(mc, lj, ti + tj, kind, s, d1.y, col_rsqrt64(s));
       Us = u.Ss * u.E + u.S * u.Es + a.p.w * u.qf * u.phis;
       Uss = u.Sss * u.E + 2.0 * u.Ss * u.Es + u.S * u.Ess + a.p.w * u.qf * u.phiss;
     } else {  // no Lennard-Jones term (and no parameters asked for)
-      const double ir = rsqrt(s), is = ir * ir;
+      const double ir = col_rsqrt64(s), is = ir * ir;
       const bool in = s <= mc.rcc2;
       const double qq = in ? a.p.w * d1.y * (kind ? mc.csf : 1.0) : 0.0;
       Us = qq * (-0.5 * ir * is + mc.c05_3);

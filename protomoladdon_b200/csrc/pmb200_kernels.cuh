@@ -1795,16 +1795,16 @@ enum DerivMode { DERIV_PARAMS = 0, DERIV_VJP = 1 };
 struct DerivTerms {
   double is, is3, is6, E, Es, Ess, S, Ss, Sss, qf, phi, phis, phiss;
 };
+// (ir: 1 / sqrt(s))
 __device__ __forceinline__ DerivTerms deriv_terms(const Fp64Consts &mc,
                                                   const double4 *__restrict__ lj64, int tab,
-                                                  int kind, double s, double qj) {
+                                                  int kind, double s, double qj, double ir) {
   DerivTerms u;
   const double4 p = lj64[tab];
   const double A = kind == 1 ? p.z : p.x;
   const double B = kind == 1 ? p.w : p.y;
   // one reciprocal square root serves both 1/s and s^-1/2 (the Coulomb
   // terms): 1/s as its square, within 2 ulp of the quotient
-  const double ir = rsqrt(s);
   u.is = ir * ir;
   u.is3 = u.is * u.is * u.is;
   u.is6 = u.is3 * u.is3;
@@ -1917,7 +1917,7 @@ k_deriv_fp64(GridParams g, Fp64Consts mc, const Stencil st, int ntypes,
               kind = excl_kind(ex, elo, ehi, sidx[j]);
               if (kind == 2) continue;
             }
-            const DerivTerms u = deriv_terms(mc, lj64, ti + mj.x, kind, s, pj.w);
+            const DerivTerms u = deriv_terms(mc, lj64, ti + mj.x, kind, s, pj.w, rsqrt(s));
             const double E = u.E, Es = u.Es, Ess = u.Ess, S = u.S, Ss = u.Ss, Sss = u.Sss;
             const double is = u.is, is3 = u.is3, is6 = u.is6;
             const double qf = u.qf, phi = u.phi, phis = u.phis, phiss = u.phiss;
@@ -2112,7 +2112,7 @@ k_deriv_fp64_half(GridParams g, Fp64Consts mc, const HalfStencil st, int slots, 
           const bool near = s <= mc.cut2 && s > 0.0;
           if (kind == 0 && near && mj.y == mi.y) kind = excl_kind(ex, elo, ehi, sidx[j]);
           if (kind != 2 && near) {
-            const DerivTerms u = deriv_terms(mc, lj64, ti + mj.x, kind, s, pj.w);
+            const DerivTerms u = deriv_terms(mc, lj64, ti + mj.x, kind, s, pj.w, rsqrt(s));
             double T = 0.0;
             if (kVjp) {
               const double4 wj = sm.w[t];
