@@ -84,15 +84,14 @@ struct pmb200_ctx {
   MixedConsts mcc{};          // the pair constants in the columns' length unit
   double col_unit = 1.0;      // that unit (A)
   int col_clusters = 0;       // upper bound of the clusters
-  size_t col_n_alloc = 0, col_slot_alloc = 0, col_ncol_alloc = 0, col_bucket_alloc = 0,
-         col_zs_alloc = 0, col_part_alloc = 0, col_lj_alloc = 0;
+  char *d_carena = nullptr;   // the column kernels' buffers and tables
+  size_t carena_bytes = 0, col_ncol_alloc = 0;
   bool col_count_zero = false;
   double *d_csq = nullptr;
   // FP64 kernels: wrapped positions (caller and slot order), a direction
   double4 *d_dpos = nullptr, *d_cspos64 = nullptr, *d_cw = nullptr;
   size_t dpos_alloc = 0, cspos64_alloc = 0, cw_alloc = 0;
   int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr, *d_icom = nullptr;
-  size_t icom_alloc = 0;
   int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_cscratch = nullptr;
   int *d_cctl = nullptr;
   unsigned char *d_ljact = nullptr;
@@ -436,11 +435,8 @@ int pull_lj(pmb200_ctx *c) {
 // The column kernels' LJ tables (in their length unit, FP32 and FP64) and, per
 // type, whether any type meets it with a non-zero entry (atoms of the other
 // types -- the hydrogens of 3-site waters -- skip the LJ arithmetic).
-int col_upload_lj(pmb200_ctx *c) {
+void col_lj_tables(const pmb200_ctx *c, double2 *l64, float4 *l32, unsigned char *act) {
   const int nt = c->ntypes, t2 = nt * nt;
-  std::vector<double2> l64(2 * t2);
-  std::vector<float4> l32(t2);
-  std::vector<unsigned char> act(nt, 0);
   const double u = c->col_unit;
   const double u6 = std::pow(u, 6.0), u12 = u6 * u6;
   for (int k = 0; k < t2; k++) {
@@ -451,11 +447,25 @@ int col_upload_lj(pmb200_ctx *c) {
                          (float)l64[t2 + k].y);
     if (p[0] != 0.0 || p[1] != 0.0 || p[2] != 0.0 || p[3] != 0.0) act[k % nt] = 1;
   }
-  CK(cudaMemcpyAsync(c->d_ljc64, l64.data(), sizeof(double2) * 2 * t2, cudaMemcpyHostToDevice,
-                     c->stream));
-  CK(cudaMemcpyAsync(c->d_ljc32, l32.data(), sizeof(float4) * t2, cudaMemcpyHostToDevice,
-                     c->stream));
-  CK(cudaMemcpyAsync(c->d_ljact, act.data(), (size_t)nt, cudaMemcpyHostToDevice, c->stream));
+}
+
+// The tables and the neighbour columns, which lie back to back in the arena.
+int col_upload(pmb200_ctx *c) {
+  const int nt = c->ntypes, t2 = nt * nt;
+  char *base = reinterpret_cast<char *>(c->d_ljc64);
+  auto at = [&](const void *p) { return (size_t)(static_cast<const char *>(p) - base); };
+  const size_t bytes = at(c->d_cst) + sizeof(short2) * (size_t)c->cst.n;
+  std::vector<double> blob((bytes + 7) / 8, 0.0);
+  char *h = reinterpret_cast<char *>(blob.data());
+  std::vector<double2> l64(2 * (size_t)t2);
+  std::vector<float4> l32(t2);
+  std::vector<unsigned char> act(nt, 0);
+  col_lj_tables(c, l64.data(), l32.data(), act.data());
+  std::memcpy(h, l64.data(), sizeof(double2) * l64.size());
+  std::memcpy(h + at(c->d_ljc32), l32.data(), sizeof(float4) * l32.size());
+  std::memcpy(h + at(c->d_ljact), act.data(), act.size());
+  std::memcpy(h + at(c->d_cst), c->cst.off, sizeof(short2) * (size_t)c->cst.n);
+  CK(cudaMemcpyAsync(base, h, bytes, cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return PMB200_OK;
 }
@@ -480,7 +490,7 @@ int upload_lj(pmb200_ctx *c) {
   CK(cudaMemcpyAsync(c->d_lj32, l32.data(), sizeof(float4) * t2, cudaMemcpyHostToDevice,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  return c->col_ok ? col_upload_lj(c) : PMB200_OK;
+  return c->col_ok ? col_upload(c) : PMB200_OK;
 }
 
 int ensure_atom_buffers(pmb200_ctx *c) {
@@ -1031,8 +1041,8 @@ int col_grow64(pmb200_ctx *c, bool w) {
     return e;
   };
   CK(grow(c->d_dpos, c->dpos_alloc, (size_t)c->n));
-  CK(grow(c->d_cspos64, c->cspos64_alloc, c->col_slot_alloc));
-  if (w) CK(grow(c->d_cw, c->cw_alloc, c->col_slot_alloc));
+  CK(grow(c->d_cspos64, c->cspos64_alloc, (size_t)c->cg.nslot));
+  if (w) CK(grow(c->d_cw, c->cw_alloc, (size_t)c->cg.nslot));
   return PMB200_OK;
 }
 
@@ -1111,51 +1121,61 @@ int col_prepare(pmb200_ctx *c) {
   const int cl = n / kColI;
   g.nparts = cl >= 16000 ? 1 : (cl >= 2500 ? 2 : (cl >= 600 ? 4 : 8));
   for (c->col_lsplit = 0; 2 << c->col_lsplit <= g.nparts;) c->col_lsplit++;
-  // buffers
-  auto grow = [&](auto *&p, size_t &have, size_t want) -> cudaError_t {
-    if (have >= want && p) return cudaSuccess;
-    have = 0;
-    const cudaError_t e = dalloc(p, want);
-    if (e == cudaSuccess) have = want;
-    return e;
-  };
+  c->cg = g;
+  // buffers, carved from one allocation (a batch's hundreds of contexts would
+  // otherwise spend their construction in the allocator); the tables last, back
+  // to back for one upload
   const size_t t2 = (size_t)c->ntypes * c->ntypes;
-  CK(grow(c->d_ipos, c->col_n_alloc, (size_t)n));
-  if (c->col_slot_alloc < (size_t)g.nslot) {
-    c->col_slot_alloc = 0;
-    CK(dalloc(c->d_cspos, (size_t)g.nslot));
-    CK(dalloc(c->d_csmeta, (size_t)g.nslot));
-    CK(dalloc(c->d_cscratch, (size_t)g.nslot));
-    CK(dalloc(c->d_csq, (size_t)g.nslot));
-    c->col_slot_alloc = (size_t)g.nslot;
+  auto carve = [&](char *base) {
+    size_t off = 0;
+    auto take = [&](auto *&p, size_t count) {
+      using T = std::remove_pointer_t<std::remove_reference_t<decltype(p)>>;
+      if (base) p = reinterpret_cast<T *>(base + off);
+      off = (off + sizeof(T) * count + 255) & ~(size_t)255;
+    };
+    take(c->d_cctl, 4);
+    take(c->d_ipos, (size_t)n);
+    take(c->d_cspos, (size_t)g.nslot);
+    take(c->d_csmeta, (size_t)g.nslot);
+    take(c->d_cscratch, (size_t)g.nslot);
+    take(c->d_csq, (size_t)g.nslot);
+    take(c->d_bucket, (size_t)g.ncol * g.cap);
+    take(c->d_zs, (size_t)g.ncol * (g.nsz + 1));
+    take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
+    take(c->d_icom, (size_t)std::max(c->nmol, 1));
+    take(c->d_ljc64, 2 * t2);
+    take(c->d_ljc32, t2);
+    take(c->d_ljact, (size_t)c->ntypes);
+    take(c->d_cst, (size_t)kColMaxCls);
+    return off;
+  };
+  const size_t want = carve(nullptr);
+  if (want > c->carena_bytes) {
+    c->carena_bytes = 0;
+    CK(dalloc(c->d_carena, want));
+    c->carena_bytes = want;
   }
-  CK(grow(c->d_ccount, c->col_ncol_alloc, (size_t)g.ncol));
-  CK(cudaMemset(c->d_ccount, 0, sizeof(int) * (size_t)g.ncol));
-  c->col_count_zero = true;
-  CK(grow(c->d_bucket, c->col_bucket_alloc, (size_t)g.ncol * g.cap));
-  CK(grow(c->d_zs, c->col_zs_alloc, (size_t)g.ncol * (g.nsz + 1)));
-  CK(grow(c->d_cpartial, c->col_part_alloc, (size_t)c->col_clusters * g.nparts * kNacc));
-  CK(grow(c->d_icom, c->icom_alloc, (size_t)std::max(c->nmol, 1)));
-  if (!c->d_cctl) CK(dalloc(c->d_cctl, 4));
+  carve(c->d_carena);
+  // (the counts keep their place: every evaluation leaves them zero)
+  if (c->col_ncol_alloc < (size_t)g.ncol) {
+    c->col_ncol_alloc = 0;
+    CK(dalloc(c->d_ccount, (size_t)g.ncol));
+    c->col_ncol_alloc = (size_t)g.ncol;
+    c->col_count_zero = false;
+  }
+  if (!c->col_count_zero) {
+    CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * c->col_ncol_alloc, c->stream));
+    c->col_count_zero = true;
+  }
   if (c->p.precision == PMB200_FP64) {  // (mixed contexts: at the first derivative)
     const int r64 = col_grow64(c, false);
     if (r64) return r64;
   }
-  if (!c->d_cst) CK(dalloc(c->d_cst, (size_t)kColMaxCls));
-  CK(cudaMemcpy(c->d_cst, c->cst.off, sizeof(short2) * (size_t)c->cst.n, cudaMemcpyHostToDevice));
-  if (c->col_lj_alloc < t2) {
-    c->col_lj_alloc = 0;
-    CK(dalloc(c->d_ljc32, t2));
-    CK(dalloc(c->d_ljc64, 2 * t2));
-    CK(dalloc(c->d_ljact, (size_t)c->ntypes));
-    c->col_lj_alloc = t2;
-  }
   c->mcc = mixed_consts(c, rc, u);
   c->col_full = c->mcc.rclj2 >= c->mcc.cut2 && c->mcc.rcc2 >= c->mcc.cut2;
-  c->cg = g;
   int r = pull_lj(c);
   if (r) return r;
-  r = col_upload_lj(c);
+  r = col_upload(c);
   if (r) return r;
   c->col_ok = true;
   release_graph(c);
@@ -1631,10 +1651,7 @@ int pmb200_destroy(pmb200_ctx *c) {
   dfree(c->d_sc_clo); dfree(c->d_sc_chi); dfree(c->d_sc_sbox); dfree(c->d_sc_corg);
   dfree(c->d_sc_sorg); dfree(c->d_sc_tasks); dfree(c->d_sc_cmol); dfree(c->d_sc_ent);
   dfree(c->d_sc_facc); dfree(c->d_sc_part);
-  dfree(c->d_ipos); dfree(c->d_cspos); dfree(c->d_csmeta); dfree(c->d_icom);
-  dfree(c->d_ccount); dfree(c->d_bucket); dfree(c->d_zs); dfree(c->d_cscratch);
-  dfree(c->d_cctl); dfree(c->d_ljact); dfree(c->d_ljc32); dfree(c->d_ljc64);
-  dfree(c->d_cpartial); dfree(c->d_csq); dfree(c->d_cst);
+  dfree(c->d_carena); dfree(c->d_ccount);
   dfree(c->d_dpos); dfree(c->d_cspos64); dfree(c->d_cw);
   if (c->h_pin_pos) cudaFreeHost(c->h_pin_pos);
   if (c->h_pin_frc) cudaFreeHost(c->h_pin_frc);
@@ -1719,6 +1736,7 @@ int pmb200_set_topology(pmb200_ctx *c, int n, const int *type, const double *q_s
   c->csf = coulomb_scaling;
   c->has_modified = modified;
   c->have_mass = mass != nullptr;
+  c->col_ok = false;  // (until prepare_kernels; the tables' sizes change)
   c->h_lj.assign(lj, lj + 4 * ntypes * ntypes);
   c->lj_dev_newer = false;
   const size_t nn = (size_t)std::max(n, 1);
@@ -1935,6 +1953,7 @@ int pmb200_set_box(pmb200_ctx *c, const double e1[3], const double e2[3], const 
   }
   if (c->vacuum) b.d = std::numeric_limits<double>::infinity();  // no images
   c->have_box = true;
+  c->col_ok = false;  // (until prepare_kernels)
   if (c->have_topo) {
     const int r = upload_lj(c);
     return r ? r : prepare_kernels(c);
@@ -2515,7 +2534,7 @@ __global__ void k_update_lj(int t2, const double *__restrict__ src, double u6, d
   if (!(isfinite(a) && isfinite(b) && isfinite(a14) && isfinite(b14))) atomicOr(err, 4);
   lj64[k] = make_double4(a, b, a14, b14);
   lj32[k] = make_float4((float)(a / u12), (float)(b / u6), (float)(a14 / u12), (float)(b14 / u6));
-  if (ljc64) {  // the column kernels' tables (col_upload_lj)
+  if (ljc64) {  // the column kernels' tables (col_upload)
     const double2 l = make_double2(a / v12, b / v6), m = make_double2(a14 / v12, b14 / v6);
     ljc64[k] = l;
     ljc64[t2 + k] = m;
@@ -3791,10 +3810,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
       l32.resize(l32.size() + t2);
       l64.resize(l64.size() + 2 * t2);
       act.resize(act.size() + c->ntypes);
-      BCK(cudaMemcpy(&l32[y.lj0], c->d_ljc32, sizeof(float4) * t2, cudaMemcpyDeviceToHost));
-      BCK(cudaMemcpy(&l64[2 * (size_t)y.lj0], c->d_ljc64, sizeof(double2) * 2 * t2,
-                     cudaMemcpyDeviceToHost));
-      BCK(cudaMemcpy(&act[y.act0], c->d_ljact, (size_t)c->ntypes, cudaMemcpyDeviceToHost));
+      col_lj_tables(c, &l64[2 * (size_t)y.lj0], &l32[y.lj0], &act[y.act0]);
       slots += c->cg.nslot;
       zs += (long long)c->cg.ncol * (c->cg.nsz + 1);
       bucket += (long long)c->cg.ncol * c->cg.cap;

@@ -40,8 +40,7 @@ constexpr int kColCap = 128;      // staged j atoms per flush
 constexpr int kColMaxCls = 256;   // neighbour-column classes
 constexpr int kColSortCap = 1536; // atoms a column sort holds in shared memory
 constexpr int kColMaxSlabs = 1024;
-constexpr int kColSortThreads = 128;
-constexpr int kColMaxParts = 8;
+constexpr int kColSortThreads = 256;
 
 struct ColGrid {
   int ncx, ncy, ncol, nsz;   // columns along x and y, slabs per column

@@ -60,6 +60,7 @@ __device__ __forceinline__ double col_rsqrt64(double x) {
 //   pair(front, a16, a8)   this lane's atom against the entry there
 //   start()                zero the j terms
 //   shift(to)              the j terms moved to the lane `to` away
+//   join(to)               the j terms of the lane `to` away added
 //   finish(a8)             the j terms (whole) added to the entry's atom
 template <bool kW, bool kSplit, class Pair>
 struct ColWalk64 {
@@ -69,22 +70,28 @@ struct ColWalk64 {
   int nl = 0, nn = 0;  // staged entries from the front, from the back
 
   template <class Tag>
-  __device__ __forceinline__ void block(Tag tag, int e0) {
-    const unsigned e = (unsigned)(e0 + (threadIdx.x & 31));
+  // half: the block's first 16 entries, four per lane group -- two lanes then
+  // meet one entry, each with its own part of the j terms, and four steps are
+  // enough (3% of the derivative kernels' time; the mixed kernel, with shorter
+  // steps, lost as much to the choice as it gained)
+  __device__ __forceinline__ void block(Tag tag, int e0, bool half) {
+    const int lane = threadIdx.x & 31;
+    const unsigned e = (unsigned)(e0 + (half ? 4 * (lane >> 3) + (lane & 3) : lane));
     unsigned a16 = sb + Lay::pos + 16 * e, a8 = sb + Lay::mg + 8 * e;
     pair.start();
 #pragma unroll 1
-    for (int h = 0; h < 4; h++) {
+    for (int h = half ? 2 : 0; h < 4; h++) {
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        const unsigned to = k == 0 ? 1u : (h & 1 ? 7u : 3u);
+        const unsigned to = k == 0 ? 1u : ((h & 1) && !half ? 7u : 3u);
         pair(tag, a16, a8);
         pair.shift((int)to);
         a16 ^= to << 4;
         a8 ^= to << 3;
       }
     }
-    pair.finish(a8);
+    if (half) pair.join(4);
+    if (!half || !(lane & 4)) pair.finish(a8);
   }
   __device__ __forceinline__ void copy(int from, int to) {
     for (unsigned h = 0; h <= Lay::half; h += Lay::half) {
@@ -105,7 +112,7 @@ struct ColWalk64 {
     __syncwarp();
     const int bn = kSplit ? nn & ~(kColBlk - 1) : 0;
     if (kSplit)
-      for (int t = 0; t < bn; t += kColBlk) block(std::false_type{}, kColCap - kColBlk - t);
+      for (int t = 0; t < bn; t += kColBlk) block(std::false_type{}, kColCap - kColBlk - t, false);
     const int r = nn - bn;
     int fn = nl & ~(kColBlk - 1);
     if (last) {
@@ -122,7 +129,7 @@ struct ColWalk64 {
       }
       __syncwarp();
     }
-    for (int t = 0; t < fn; t += kColBlk) block(std::true_type{}, t);
+    for (int t = 0; t < fn; t += kColBlk) block(std::true_type{}, t, last && nl - t <= 16);
     __syncwarp();
     if (last) {
       nl = nn = 0;
@@ -336,6 +343,11 @@ struct ColPair64 {
     jy = __shfl_xor_sync(0xffffffffu, jy, to);
     jz = __shfl_xor_sync(0xffffffffu, jz, to);
   }
+  __device__ __forceinline__ void join(int to) {
+    jx += __shfl_xor_sync(0xffffffffu, jx, to);
+    jy += __shfl_xor_sync(0xffffffffu, jy, to);
+    jz += __shfl_xor_sync(0xffffffffu, jz, to);
+  }
   __device__ __forceinline__ void finish(unsigned a8) {
     const int r = lds1(a8 + 4);
     fix2_add_rank(acc, A.n, r, 0, jx, A.err);
@@ -497,6 +509,14 @@ struct ColDeriv64 {
       jz = __shfl_xor_sync(0xffffffffu, jz, to);
     }
     if (kParams) jq = __shfl_xor_sync(0xffffffffu, jq, to);
+  }
+  __device__ __forceinline__ void join(int to) {
+    if (kVjp) {
+      jx += __shfl_xor_sync(0xffffffffu, jx, to);
+      jy += __shfl_xor_sync(0xffffffffu, jy, to);
+      jz += __shfl_xor_sync(0xffffffffu, jz, to);
+    }
+    if (kParams) jq += __shfl_xor_sync(0xffffffffu, jq, to);
   }
   __device__ __forceinline__ void finish(unsigned a8) {
     const int r = lds1(a8 + 4);
