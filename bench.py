@@ -64,13 +64,13 @@ sys.path.insert(0, ROOT)
 DT_FS = 1.0
 FLOPS_PER_PAIR = 81          # algorithmic flops per unique in-cutoff pair
 BYTES_PER_ATOM = 84          # algorithmic HBM bytes per atom per evaluation
-KERNELS_PER_STEP = 7         # kick_drift_settle, cell_index, scan, scatter, rank_gather,
-                             # pair, finalize_reduce (forces and energy sums)
+KERNELS_PER_STEP = 5         # kick_drift_settle, col_index, col_sort, col_pair,
+                             # col_finalize_reduce (forces and energy sums)
 KERNELS_PER_STEP_CLUSTERS = 13  # kick_drift_settle, sc_index, scan, scatter, rank_gather,
                              # sc_columns, sc_build, sc_list, sc_tasks, sc_pair,
                              # sc_finalize, sc_reduce1, reduce2
 # ncu summaries holding each energy launch's DRAM bytes (traffic_bytes_per_launch)
-TRAFFIC_PROFILE = {"search": "pair_mixed_water41k.md", "clusters": "pair_clusters_water41k.md",
+TRAFFIC_PROFILE = {"search": "pair_columns_water41k.md", "clusters": "pair_clusters_water41k.md",
                    "tiles": None}
 WORKLOAD = ("water box: 41,472 atoms (13,824 TIP3P-geometry waters, 24^3 lattice, "
             "box 74.496 A), LJ C2 switch 9-10 A + Coulomb C1 cutoff 10 A, leapfrog 1 fs")
@@ -140,7 +140,7 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------------------
-def committed_traffic(name="pair_mixed_water41k.md"):
+def committed_traffic(name="pair_columns_water41k.md"):
     """Pair-kernel DRAM bytes per launch from a committed ncu summary."""
     path = os.path.join(ROOT, "profiles", name)  # ncu summary
     try:
@@ -320,7 +320,7 @@ def run_ours(args):
 
     def tune(force):
         """pmb200_autotune on the start positions: the grid's cell size, the
-        pair kernel and its warps per i-cell, applied to the context (or the
+        pair kernel and the cell kernel's warps per i-cell, applied to the context (or the
         pair kernel --pair-kernel names, untuned)."""
         pos = torch.tensor(s["pos"], dtype=torch.float64, device=dev)
         if args.pair_kernel != "auto" and force.precision == "mixed":
@@ -499,8 +499,7 @@ def run_ours(args):
                 "forces_only_ms_per_step": other[2], "forces_only_pair_kernel_ms": other[3],
                 "pair_kernel_fp32_frac": (FLOPS_PER_PAIR * pairs / (other[1] * 1e-3) / 1e12
                                           / peak) if peak else None,
-                "note": "the same device steps on the supercluster kernel: its pair kernel is "
-                        "faster, its per-step list build costs more; the autotuner keeps "
+                "note": "the same device steps on the supercluster kernel; the autotuner keeps "
                         "the faster whole step"}} if other else {}),
             "gpu_launches": (KERNELS_PER_STEP_CLUSTERS if kern_e == "clusters"
                              else KERNELS_PER_STEP) * args.steps,
@@ -513,9 +512,9 @@ def run_ours(args):
                             "pair_kernel_ms": fp64[1],
                             "mixed_speedup": t64 / ms_step,
                             "pair_kernel_speedup": fp64[1] / mean_k,
-                            "kernel": "k_pair_fp64_half: the mixed kernel's half-shell task "
-                                      "split and box culling in FP64, each pair once, exact "
-                                      "fixed-point force sums; the same device steps"}
+                            "kernel": "k_col_pair64: the column kernels' walk in FP64, each "
+                                      "pair once, exact fixed-point force sums; the same "
+                                      "device steps"}
         if world == 1 and not args.skip_cpu:
             cpu_steps = args.cpu_steps
             t_cpu, kind = cpu_reference_time(s, cpu_steps)
