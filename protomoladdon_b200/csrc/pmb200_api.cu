@@ -3545,7 +3545,8 @@ struct pmb200_batch {
   int4 *d_tasks = nullptr;
   int *d_rows_start = nullptr, *d_rows = nullptr;
   // column kernels (every system periodic and orthogonal)
-  bool col = false, col_full = true, col_mod = false, col_dirty = false;
+  bool col = false, col_full = true, col_mod = false, col_dirty = false,
+       col_small = true;
   std::vector<ColBatchSys> h_col;
   std::vector<int> col_parts;   // each context's own number of parts
   int ncol = 0;
@@ -3713,10 +3714,14 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
     k_col_index_batch<<<(N + 255) / 256, 256, 0, st>>>(N, d_pos, b->d_col, b->d_atom_sys, b->d_q,
                                                        b->d_ipos, b->d_ccount, b->d_bucket,
                                                        b->d_facc, b->d_err);
-    k_col_sort_batch<<<b->ncol, kColSortThreads, 0, st>>>(
-        b->d_col, b->d_col_sys, b->d_ipos, b->d_ccount, b->d_bucket, b->d_type, b->d_mol,
-        b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_sidx, b->d_zs, b->d_scratch,
-        b->d_ctl);
+    auto sort = [&](auto kernel, int threads) {
+      kernel<<<b->ncol, threads, 0, st>>>(
+          b->d_col, b->d_col_sys, b->d_ipos, b->d_ccount, b->d_bucket, b->d_type, b->d_mol,
+          b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_sidx, b->d_zs,
+          b->d_scratch, b->d_ctl);
+    };
+    if (b->col_small) sort(k_col_sort_batch<kColSortThreadsS, kColSortCapS>, kColSortThreadsS);
+    else sort(k_col_sort_batch<kColSortThreads, kColSortCap>, kColSortThreads);
     BCK(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
     ColArrays a{};
     ColBatchLaunch l = batch_col_launch(b, energy, virial, a);
@@ -3806,6 +3811,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
       b->col_parts.back() = c->cg.nparts;
       b->col_full = b->col_full && c->col_full;
       b->col_mod = b->col_mod || c->has_modified;
+      b->col_small = b->col_small && c->cg.cap <= kColSortCapS && c->cg.ncol <= 1024;
       const size_t t2 = (size_t)c->ntypes * c->ntypes;
       l32.resize(l32.size() + t2);
       l64.resize(l64.size() + 2 * t2);
