@@ -1196,7 +1196,7 @@ bool columns_apply(const pmb200_ctx *c, unsigned flags) {
 
 // (d_w: a direction to gather beside the FP64 positions; fp64: these wanted)
 int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
-                     unsigned long long *clear, int nclear = 3, bool fp64 = false,
+                     unsigned long long *clear, bool molvir, int nclear = 3, bool fp64 = false,
                      const double *d_w = nullptr) {
   const int n = c->n;
   const ColGrid &g = c->cg;
@@ -1207,9 +1207,11 @@ int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
   if (!c->col_count_zero)
     CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * (size_t)g.ncol, st));
   c->col_count_zero = false;
-  launch_k(k_col_index, (unsigned)((n + 255) / 256), 256, 0, st, false, n, d_pos, g,
+  const ColMols mols{molvir ? c->nmol : 0, c->d_mstart, c->d_matoms, c->d_mass, c->d_icom};
+  launch_k(mols.n ? k_col_index<true> : k_col_index<false>,
+           (unsigned)((n + 255) / 256 + (mols.n + 255) / 256), 256, 0, st, false, n, d_pos, g,
            (const double *)c->d_q, c->d_ipos, c->d_ccount, c->d_bucket, clear,
-           clear ? nclear : 0, c->d_err, fp64 ? c->d_dpos : nullptr);
+           clear ? nclear : 0, c->d_err, fp64 ? c->d_dpos : nullptr, mols);
   launch_k(k_col_sort, (unsigned)g.ncol, kColSortThreads, 0, st, true, n, g,
            (const int4 *)c->d_ipos, (const int *)c->d_ccount, (const int *)c->d_bucket,
            (const int *)c->d_type, (const int *)c->d_mol, (const unsigned char *)c->d_ljact,
@@ -1289,13 +1291,9 @@ int launch_eval_columns(pmb200_ctx *c, const double *d_pos, double *d_forces, do
   const bool energy = (flags & PMB200_ENERGY) != 0;
   const bool virial = (flags & (PMB200_VIRIAL | PMB200_MOLVIRIAL)) != 0;
   const bool mixed = c->p.precision == PMB200_MIXED;
-  int r = launch_col_build(c, d_pos, st, c->d_facc, mixed ? 3 : 8, !mixed);
+  int r = launch_col_build(c, d_pos, st, c->d_facc, (flags & PMB200_MOLVIRIAL) != 0,
+                           mixed ? 3 : 8, !mixed);
   if (r) return r;
-  if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
-    k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms, c->d_mass,
-                                                  d_pos, c->d_com);
-    k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
-  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(st, &cap));
   const bool timed = c->timing && cap == cudaStreamCaptureStatusNone;
@@ -2284,13 +2282,8 @@ int pmb200_shard_eval_device(pmb200_ctx *c, const double *d_pos, int shard, int 
   const int hi = (int)((long long)g.ncell * (shard + 1) / nshards);
   unsigned long long *facc = reinterpret_cast<unsigned long long *>(d_facc);
   if (c->col_ok) {
-    rc = launch_col_build(c, d_pos, st, facc);
+    rc = launch_col_build(c, d_pos, st, facc, (flags & PMB200_MOLVIRIAL) != 0);
     if (rc) return rc;
-    if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
-      k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms,
-                                                    c->d_mass, d_pos, c->d_com);
-      k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
-    }
     const ColShare share{shard, shard + 1, nshards};
     rc = launch_col_pair(c, flags, st, true, share, facc);
     if (rc) return rc;
@@ -2394,7 +2387,8 @@ static int launch_deriv(pmb200_ctx *c, int mode, const double *d_pos, const doub
     }
   }
   if (col) {
-    int r = launch_col_build(c, d_pos, st, c->d_facc, 8, true, mode == DERIV_VJP ? d_w : nullptr);
+    int r = launch_col_build(c, d_pos, st, c->d_facc, false, 8, true,
+                             mode == DERIV_VJP ? d_w : nullptr);
     if (r) return r;
     Col64Launch l = col64_launch(c, true);
     l.tpart = c->d_tpart;
@@ -2791,13 +2785,8 @@ int pmb200_eval_cells(pmb200_ctx *c, const double *pos, double *forces, double *
   if (mixed && c->col_ok) {
     // column kernels: the share of the clusters that the range is of the cells
     const ColShare share{cell_lo, cell_hi, g.ncell};
-    rc = launch_col_build(c, c->d_hpos, st, c->d_facc);
+    rc = launch_col_build(c, c->d_hpos, st, c->d_facc, (flags & PMB200_MOLVIRIAL) != 0);
     if (rc) return rc;
-    if ((flags & PMB200_MOLVIRIAL) && c->nmol > 0) {
-      k_com<<<(c->nmol + 127) / 128, 128, 0, st>>>(c->nmol, c->d_mstart, c->d_matoms,
-                                                    c->d_mass, c->d_hpos, c->d_com);
-      k_col_com<<<(c->nmol + 255) / 256, 256, 0, st>>>(c->nmol, c->d_com, c->cg, c->d_icom);
-    }
     rc = launch_col_pair(c, flags, st, true, share, c->d_facc);
     if (rc) return rc;
     k_col_finalize<false><<<(c->n + 255) / 256, 256, 0, st>>>(

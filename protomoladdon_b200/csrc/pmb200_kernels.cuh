@@ -2313,13 +2313,12 @@ k_reduce_columns(int rows, int cols, const double *__restrict__ part,
 // (mass-weighted, Kahan-compensated like molecularCenterOfMass,
 // protomol/src/protomol/topology/TopologyUtilities.cpp:645-672).
 // ---------------------------------------------------------------------------
-static __global__ void k_com(int nmol, const int *__restrict__ mstart, const int *__restrict__ matoms,
-                      const double *__restrict__ mass, const double *__restrict__ pos,
-                      double *__restrict__ com) {
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nmol) return;
-  const int lo = mstart[m], hi = mstart[m + 1];
-  if (lo == hi) { com[3 * m] = com[3 * m + 1] = com[3 * m + 2] = 0.0; return; }
+__device__ __forceinline__ void molecule_centre(const int *__restrict__ matoms,
+                                                const double *__restrict__ mass,
+                                                const double *__restrict__ pos, int lo, int hi,
+                                                double com[3]) {
+  com[0] = com[1] = com[2] = 0.0;
+  if (lo == hi) return;
   int a = matoms[lo];
   double w = mass[a], sw = w;
   double c[3], e[3] = {0, 0, 0};
@@ -2336,7 +2335,17 @@ static __global__ void k_com(int nmol, const int *__restrict__ mstart, const int
       c[k] = tt;
     }
   }
-  for (int k = 0; k < 3; k++) com[3 * m + k] = c[k] / sw;
+  for (int k = 0; k < 3; k++) com[k] = c[k] / sw;
+}
+
+static __global__ void k_com(int nmol, const int *__restrict__ mstart, const int *__restrict__ matoms,
+                      const double *__restrict__ mass, const double *__restrict__ pos,
+                      double *__restrict__ com) {
+  int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= nmol) return;
+  double c[3];
+  molecule_centre(matoms, mass, pos, mstart[m], mstart[m + 1], c);
+  for (int k = 0; k < 3; k++) com[3 * m + k] = c[k];
 }
 
 // Deterministic two-stage reduction of the per-cell partials.  Stage 1:
