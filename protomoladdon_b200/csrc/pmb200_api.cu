@@ -1,12 +1,15 @@
 // libpmb200: host side of the C ABI declared in include/pmb200.h.
 //
 // One context = one periodic system on one GPU: device copies of the
-// topology, the cell grid for the current box, per-evaluation buffers and a
-// CUDA stream.  An evaluation is
+// topology, the grids for the current box, per-evaluation buffers and a CUDA
+// stream.  An evaluation in an orthogonal periodic box (FP64: without virials) is
+//   k_col_index -> k_col_sort -> k_col_pair | k_col_pair64 -> k_col_finalize*
+// (pmb200_columns.cuh); in general cells, in vacuum, for FP64 virials and with
+// another pair kernel selected it is
 //   k_cell_index -> k_scan -> k_scatter -> k_rank_gather   (counting sort)
-//   k_pair_mixed | k_pair_fp64                            (forces, partials)
-//   [k_com -> k_molvir] -> k_reduce                        (energies, virial)
-// all on the context's stream.
+//   k_pair_mixed | k_pair_fp64_half | ...                  (forces, partials)
+//   k_finalize -> k_reduce                                 (energies, virial)
+// all on the caller's stream.
 #include "../../include/pmb200.h"
 #include "pmb200_kernels.cuh"
 #include "pmb200_tiles.cuh"
@@ -90,7 +93,6 @@ struct pmb200_ctx {
   double *d_csq = nullptr;
   // FP64 kernels: wrapped positions (caller and slot order), a direction
   double4 *d_dpos = nullptr, *d_cspos64 = nullptr, *d_cw = nullptr;
-  size_t dpos_alloc = 0, cspos64_alloc = 0, cw_alloc = 0;
   int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr, *d_icom = nullptr;
   int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_cscratch = nullptr;
   int *d_cctl = nullptr;
@@ -135,7 +137,8 @@ struct pmb200_ctx {
   int n_alloc = 0;
   int *d_cell_of = nullptr, *d_slot = nullptr, *d_tmp = nullptr, *d_sidx = nullptr;
   float4 *d_rel32 = nullptr, *d_spos32 = nullptr;
-  float4 *d_rel_lo = nullptr, *d_spos_lo = nullptr;  // FP32 coordinate residuals
+  float4 *d_rel_lo = nullptr, *d_spos_lo = nullptr;  // FP32 coordinate residuals (one allocation)
+  size_t slot_room = 0;  // slots that d_spos32, d_spos64 and (as double4) d_rel_lo hold
   double4 *d_rel64 = nullptr, *d_spos64 = nullptr;
   int2 *d_smeta = nullptr;
   // force accumulator, sorted order: [3][n] 2^-32 quanta (mixed) or [6][n]
@@ -500,12 +503,17 @@ int ensure_atom_buffers(pmb200_ctx *c) {
   CK(dalloc(c->d_slot, n));
   CK(dalloc(c->d_tmp, n));
   CK(dalloc(c->d_sidx, n));
+  // (with room for the column kernels' slots, which share some of them: an
+  // evaluation runs on one kind of kernel)
+  const size_t slots = n + n / 4 + 64;
+  c->slot_room = 0;
   CK(dalloc(c->d_rel32, n));
-  CK(dalloc(c->d_spos32, n));
-  CK(dalloc(c->d_rel_lo, n));
-  CK(dalloc(c->d_spos_lo, n));
+  CK(dalloc(c->d_spos32, slots));
+  CK(dalloc(c->d_rel_lo, 2 * slots));
+  c->d_spos_lo = c->d_rel_lo + slots;
   CK(dalloc(c->d_rel64, n));
-  CK(dalloc(c->d_spos64, n));
+  CK(dalloc(c->d_spos64, slots));
+  c->slot_room = slots;
   CK(dalloc(c->d_smeta, n));
   CK(dalloc(c->d_facc, 8 * n));  // FP64 forces: 6 words per atom; derivatives: 8
   CK(dalloc(c->d_cblo, n));
@@ -1031,21 +1039,6 @@ int launch_eval_clusters(pmb200_ctx *c, const double *d_pos, double *d_forces, d
   return PMB200_OK;
 }
 
-// The FP64 column kernels' buffers (w: and a direction's).
-int col_grow64(pmb200_ctx *c, bool w) {
-  auto grow = [&](double4 *&p, size_t &have, size_t want) -> cudaError_t {
-    if (have >= want && p) return cudaSuccess;
-    have = 0;
-    const cudaError_t e = dalloc(p, want);
-    if (e == cudaSuccess) have = want;
-    return e;
-  };
-  CK(grow(c->d_dpos, c->dpos_alloc, (size_t)c->n));
-  CK(grow(c->d_cspos64, c->cspos64_alloc, (size_t)c->cg.nslot));
-  if (w) CK(grow(c->d_cw, c->cw_alloc, (size_t)c->cg.nslot));
-  return PMB200_OK;
-}
-
 // The column kernels' grid, neighbour columns, constants, tables and buffers
 // for the current box and topology (col_ok = false where they do not apply:
 // general cells and vacuum; the cell kernels then run).
@@ -1122,9 +1115,18 @@ int col_prepare(pmb200_ctx *c) {
   g.nparts = cl >= 16000 ? 1 : (cl >= 2500 ? 2 : (cl >= 600 ? 4 : 8));
   for (c->col_lsplit = 0; 2 << c->col_lsplit <= g.nparts;) c->col_lsplit++;
   c->cg = g;
-  // buffers, carved from one allocation (a batch's hundreds of contexts would
-  // otherwise spend their construction in the allocator); the tables last, back
-  // to back for one upload
+  // buffers: the cell kernels' where they are large enough, the rest carved from
+  // one allocation (a batch's hundreds of contexts would otherwise spend their
+  // construction in the allocator); the tables last, back to back for one upload
+  const bool room = (size_t)g.nslot <= c->slot_room;
+  const bool rows = (long long)c->col_clusters * g.nparts <=
+                    (long long)c->ncell_alloc * kMaxCellSlots;
+  c->d_ipos = reinterpret_cast<int4 *>(c->d_rel32);
+  c->d_dpos = c->d_rel64;
+  c->d_cspos = reinterpret_cast<int4 *>(c->d_spos32);
+  c->d_cspos64 = c->d_spos64;
+  c->d_cw = reinterpret_cast<double4 *>(c->d_rel_lo);
+  c->d_cpartial = c->d_partial;
   const size_t t2 = (size_t)c->ntypes * c->ntypes;
   auto carve = [&](char *base) {
     size_t off = 0;
@@ -1134,14 +1136,17 @@ int col_prepare(pmb200_ctx *c) {
       off = (off + sizeof(T) * count + 255) & ~(size_t)255;
     };
     take(c->d_cctl, 4);
-    take(c->d_ipos, (size_t)n);
-    take(c->d_cspos, (size_t)g.nslot);
+    if (!room) {
+      take(c->d_cspos, (size_t)g.nslot);
+      take(c->d_cspos64, (size_t)g.nslot);
+      take(c->d_cw, (size_t)g.nslot);
+    }
     take(c->d_csmeta, (size_t)g.nslot);
     take(c->d_cscratch, (size_t)g.nslot);
     take(c->d_csq, (size_t)g.nslot);
     take(c->d_bucket, (size_t)g.ncol * g.cap);
     take(c->d_zs, (size_t)g.ncol * (g.nsz + 1));
-    take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
+    if (!rows) take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
     take(c->d_icom, (size_t)std::max(c->nmol, 1));
     take(c->d_ljc64, 2 * t2);
     take(c->d_ljc32, t2);
@@ -1166,10 +1171,6 @@ int col_prepare(pmb200_ctx *c) {
   if (!c->col_count_zero) {
     CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * c->col_ncol_alloc, c->stream));
     c->col_count_zero = true;
-  }
-  if (c->p.precision == PMB200_FP64) {  // (mixed contexts: at the first derivative)
-    const int r64 = col_grow64(c, false);
-    if (r64) return r64;
   }
   c->mcc = mixed_consts(c, rc, u);
   c->col_full = c->mcc.rclj2 >= c->mcc.cut2 && c->mcc.rcc2 >= c->mcc.cut2;
@@ -1200,10 +1201,6 @@ int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
                      const double *d_w = nullptr) {
   const int n = c->n;
   const ColGrid &g = c->cg;
-  if (fp64) {
-    const int r = col_grow64(c, d_w != nullptr);
-    if (r) return r;
-  }
   if (!c->col_count_zero)
     CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * (size_t)g.ncol, st));
   c->col_count_zero = false;
@@ -1639,7 +1636,7 @@ int pmb200_destroy(pmb200_ctx *c) {
   dfree(c->d_lj32); dfree(c->d_lj64); dfree(c->d_ljtab); dfree(c->d_cblo); dfree(c->d_cbhi);
   dfree(c->d_count); dfree(c->d_start); dfree(c->d_err); dfree(c->d_partial);
   dfree(c->d_cell_of); dfree(c->d_slot); dfree(c->d_tmp); dfree(c->d_sidx);
-  dfree(c->d_rel32); dfree(c->d_spos32); dfree(c->d_rel_lo); dfree(c->d_spos_lo); dfree(c->d_rel64); dfree(c->d_spos64);
+  dfree(c->d_rel32); dfree(c->d_spos32); dfree(c->d_rel_lo); dfree(c->d_rel64); dfree(c->d_spos64);
   dfree(c->d_smeta); dfree(c->d_com); dfree(c->d_facc);
   dfree(c->d_tpart); dfree(c->d_gq); dfree(c->d_glj); dfree(c->d_wsorted);
   dfree(c->d_pairs); dfree(c->d_out); dfree(c->d_red); dfree(c->d_redctr); dfree(c->d_widx); dfree(c->d_fidx);
@@ -1650,7 +1647,6 @@ int pmb200_destroy(pmb200_ctx *c) {
   dfree(c->d_sc_sorg); dfree(c->d_sc_tasks); dfree(c->d_sc_cmol); dfree(c->d_sc_ent);
   dfree(c->d_sc_facc); dfree(c->d_sc_part);
   dfree(c->d_carena); dfree(c->d_ccount);
-  dfree(c->d_dpos); dfree(c->d_cspos64); dfree(c->d_cw);
   if (c->h_pin_pos) cudaFreeHost(c->h_pin_pos);
   if (c->h_pin_frc) cudaFreeHost(c->h_pin_frc);
   if (c->h_pin_out) cudaFreeHost(c->h_pin_out); dfree(c->d_hpos); dfree(c->d_hfrc);
@@ -1893,6 +1889,7 @@ int pmb200_set_box(pmb200_ctx *c, const double e1[3], const double e2[3], const 
   c->stencil = Stencil{};
   for (size_t r = 0; r < c->rows.size(); r++) c->stencil.rows[r] = c->rows[r];
   if (c->ncell_alloc < g.ncell) {
+    c->col_ok = false;  // (may share d_partial)
     CK(dalloc(c->d_count, (size_t)g.ncell));
     CK(cudaMemset(c->d_count, 0, sizeof(int) * (size_t)g.ncell));
     c->count_zero = true;
