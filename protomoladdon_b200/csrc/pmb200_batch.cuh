@@ -1,7 +1,10 @@
 // Batched evaluation of many independent periodic systems of uneven size:
 // one counting sort over every atom of the batch, one persistent pair
 // kernel over a task list (system, cell, part of the cell's stencil), one
-// fixed-point finalize and one per-system reduction.
+// fixed-point finalize and one per-system reduction.  (Batches whose systems all
+// have column grids run the column kernels' batch forms, pmb200_columns.cuh;
+// these serve the rest: a vacuum system among them, or a batch beyond the column
+// layout's index range.)
 //
 // Layout in HBM (N atoms and C cells over all systems, systems back to back):
 //   sys[S]            BatchSys: each system's grid, constants, offsets

@@ -1,5 +1,7 @@
 // Device kernels of libpmb200: cell build (counting sort), the mixed-precision
-// and FP64 cell-pair force kernels, reductions and the leapfrog update.
+// and FP64 cell-pair force kernels, reductions and the leapfrog update.  The pair
+// kernels here serve what the column kernels (pmb200_columns.cuh) do not: general
+// cells, vacuum, FP64 virials, the no-allocation entry.
 //
 // Data layout in HBM (per context, n atoms, C cells, x fastest):
 //   cell_of[n]        int    cell id of each atom (original order)
@@ -1517,8 +1519,8 @@ k_pair_fp64(GridParams g, Fp64Consts mc, const Stencil st, int ntypes, const dou
 }
 
 // ---------------------------------------------------------------------------
-// FP64 pair kernel on the half shell (the evaluation kernel of FP64
-// contexts): the mixed kernel's task split -- one warp per block, each warp
+// FP64 pair kernel on the half shell (FP64 contexts where the column kernels do
+// not serve: virials, general cells, vacuum): the mixed kernel's task split -- one warp per block, each warp
 // one i-cell and one share of the half-shell cell offsets (the same
 // HalfStencil; home-cell pairs taken for i < j) -- with fp64_pair's
 // arithmetic and each pair evaluated once, its force added to both atoms
