@@ -659,7 +659,7 @@ def run_large(args):
     line["e2e"] = {"value": cut["pairs_per_eval"] / (cut["e2e_ms"] * 1e-3) / 1e9,
                    "unit": "Gpairs/s", "ms_per_step": cut["e2e_ms"],
                    "h2d_bytes_per_step": 24 * n, "d2h_bytes_per_step": 24 * n + 168}
-    line["gpu_launches"] = 6 * args.steps  # cell_index, scan, scatter, rank_gather, pair, finalize
+    line["gpu_launches"] = 4 * args.steps  # col_index, col_sort, col_pair, col_finalize
     line["clocks"] = clocks
     if not args.skip_accuracy:
         from oracle import oracle as O
@@ -920,12 +920,12 @@ def run_batch(args):
         "pair_kernel_ms": k_ms,
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak else None,
-                     "traffic": committed_traffic("pair_mixed_batch_512boxes.md"),
+                     "traffic": committed_traffic("pair_columns_batch_512boxes.md"),
                      "peak_source": "FP32 FMA throughput measured in this run"},
         "e2e": {"value": pairs / statistics.mean(e2e) / 1e9, "unit": "Gpairs/s",
                 "ms_per_step": statistics.mean(e2e) * 1e3,
                 "h2d_bytes_per_step": 24 * N, "d2h_bytes_per_step": 24 * N},
-        "gpu_launches": 6 * args.steps,  # cell_index, scan, scatter, rank_gather, pair, finalize
+        "gpu_launches": 4 * args.steps,  # col_index, col_sort, col_pair, col_finalize
         "clocks": clocks,
     }
     if not args.skip_cpu:
@@ -1036,7 +1036,7 @@ def run_diff(args):
         "config": {"workload": DIFF_WORKLOAD, "step": "one Hessian-vector product (41k box)",
                    "l2": "not flushed: derivative passes run back to back as in an "
                          "optimizer loop, the ~6 MB working set staying in L2"},
-        "systems": res, "gpu_launches": 32 * 6, "clocks": clocks,
+        "systems": res, "gpu_launches": 32 * 4, "clocks": clocks,
         "e2e": {"value": big["hvp_per_s"], "unit": "HVP/s", "h2d_bytes_per_step": 0,
                 "d2h_bytes_per_step": 0},
     }
