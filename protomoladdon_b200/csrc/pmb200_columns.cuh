@@ -1042,12 +1042,18 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
 #ifndef PMB200_COL_BLOCKS
 #define PMB200_COL_BLOCKS 24
 #endif
+#ifndef PMB200_COL_BLOCKS_V
+// with virials (15,009 atoms with both, 12 / 13 / 14 / 16 blocks: 81.3 / 77.0 / 75.3 /
+// 75.3 us an evaluation; the Ewald form 77.7 / 69.4 / 69.5 / 70.6)
+#define PMB200_COL_BLOCKS_V 14
+#endif
 #ifndef PMB200_COL_BLOCKS_E
 #define PMB200_COL_BLOCKS_E 20
 #endif
 template <int kForm, bool kEnergy, bool kVirial, bool kMolVir, bool kFull, bool kMod, bool kGlobalLj>
-__global__ void __launch_bounds__(32, kVirial ? 12 : (kEnergy ? PMB200_COL_BLOCKS_E
-                                                              : PMB200_COL_BLOCKS))
+__global__ void __launch_bounds__(32, kVirial   ? PMB200_COL_BLOCKS_V
+                                      : kEnergy ? PMB200_COL_BLOCKS_E
+                                                : PMB200_COL_BLOCKS)
 k_col_pair(const ColGrid g, const MixedConsts mc, int ntypes, const float4 *__restrict__ lj32,
            const double2 *__restrict__ lj64, const ColArrays A, const int *__restrict__ ctl,
            int *__restrict__ count, int lsplit, ColShare share,
@@ -1243,8 +1249,9 @@ k_col_sort_batch(const ColBatchSys *__restrict__ sys, const int *__restrict__ co
 // Dynamic shared memory: the warp's entries, the system, its LJ tables (at most
 // lj_max type pairs).
 template <int kForm, bool kEnergy, bool kVirial, bool kFull, bool kMod>
-__global__ void __launch_bounds__(32, kVirial ? 12 : (kEnergy ? PMB200_COL_BLOCKS_E
-                                                              : PMB200_COL_BLOCKS))
+__global__ void __launch_bounds__(32, kVirial   ? PMB200_COL_BLOCKS_V
+                                      : kEnergy ? PMB200_COL_BLOCKS_E
+                                                : PMB200_COL_BLOCKS)
 k_col_pair_batch(const ColBatchSys *__restrict__ sys, const int4 *__restrict__ tasks, int ntasks,
                  int *__restrict__ counter, const short2 *__restrict__ st,
                  const float4 *__restrict__ lj32, const double2 *__restrict__ lj64,
