@@ -682,6 +682,20 @@ __device__ __forceinline__ void col_search(const ColGrid &g, const ColArrays &A,
 constexpr float kColFix = 4294967296.0f;        // 2^32 per unit force
 constexpr float kColForceLim = 1.0e9f;          // summed force component (unit force)
 
+// Whether the last flush of a walk with at most `most` staged entries overwrites
+// none that it moves: the back's rest goes behind the front entries, the filler up
+// to the next whole block behind it (no barrier orders the lanes in between).
+constexpr bool col_last_flush_apart(int most) {
+  for (int nl = 0; nl <= most; nl++)
+    for (int nn = 0; nl + nn <= most; nn++) {
+      const int r = nn % kColBlk, end = (nl + r + kColBlk - 1) / kColBlk * kColBlk;
+      if (r > 0 && end > kColCap - nn) return false;
+    }
+  return true;
+}
+static_assert(col_last_flush_apart(kColCap - 32) && !col_last_flush_apart(kColCap),
+              "a full buffer needs a flush of its whole blocks before the last one");
+
 // One warp's shared memory: kColCap staged entries -- fractions and charge (16
 // bytes), {meta, force offset} (8), for the exact energies the FP64 charge (8), for
 // the molecular virial the molecule's centre (16) -- then the cluster's molecules
@@ -925,6 +939,9 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
       atomicAdd(f + 2 * (size_t)A.n, (unsigned long long)__float2ll_rn(jz * kColFix));
     }
   };
+  // (no lane writes an entry that another still reads: what a flush moves and what
+  // it overwrites lie apart, in the last one because at most kColCap - 32 entries
+  // are left when it comes)
   auto copy_entry = [&](int from, int to) {
     sts4(sb + Lay::pos + 16 * to, lds4(sb + Lay::pos + 16 * from));
     const int2 m = lds2(sb + Lay::mg + 8 * from);
@@ -1003,7 +1020,14 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
         }
         nl += __popc(kf);
         nn += __popc(kb);
-        if (nl + nn > kColCap - 32 || last) flush(last);
+        // (a fuller buffer empties its whole blocks before the last flush, so that
+        // the rest moved to the front and the filler behind it end below the first
+        // entry to be moved)
+        bool fuller;
+        do {
+          fuller = nl + nn > kColCap - 32;
+          if (fuller || last) flush(last && !fuller);
+        } while (fuller && last);
       });
 
   // i forces over the lane groups, one component per group

@@ -93,6 +93,7 @@ struct ColWalk64 {
     if (half) pair.join(4);
     if (!half || !(lane & 4)) pair.finish(a8);
   }
+  // (what a flush moves and what it overwrites lie apart, see col_task)
   __device__ __forceinline__ void copy(int from, int to) {
     for (unsigned h = 0; h <= Lay::half; h += Lay::half) {
       const double2 d = lds2d(sb + Lay::pos + 16 * from + h);
@@ -235,7 +236,11 @@ __device__ __forceinline__ void col_search64(const ColGrid &g, const ColArrays &
         }
         walk.nl += __popc(kf);
         walk.nn += __popc(kb);
-        if (walk.nl + walk.nn > kColCap - 32 || last) walk.flush(last);
+        bool fuller;  // (see col_task)
+        do {
+          fuller = walk.nl + walk.nn > kColCap - 32;
+          if (fuller || last) walk.flush(last && !fuller);
+        } while (fuller && last);
       });
 }
 

@@ -2,8 +2,8 @@
 shapes where their layout has edges: clusters of 8 atoms and blocks of 32 staged
 ones that do not fill, boxes of exactly two cutoffs, columns that are their own
 opposite, columns whose atoms overflow their bucket or the sort's shared memory,
-clusters taller than the cutoff, exclusion lists longer than a warp -- against
-the FP64 oracle.
+clusters taller than the cutoff, exclusion lists longer than a warp, a buffer that
+is nearly full at the end -- against the FP64 oracle.
 
 Tolerances: forces 1e-5 RMS relative (the mixed kernels' bound; FP32 pair
 arithmetic leaves about 1e-6); energies 1e-6 of the pair magnitudes, about
@@ -76,6 +76,26 @@ def _unwrapped(s):
     return s
 
 
+def _ball(n, light):
+    """n single atoms on a jittered 1.9 A lattice inside one column, each within
+    the cutoff of all others of the lowest cluster; `light` of them without a
+    Lennard-Jones term.  The lowest cluster stages 7 + n - 8 atoms, at most 96 of
+    them before its last round: the buffer is fuller than a last flush may find it."""
+    s = _waters(1, (16.5, 16.5, 100.0))
+    rng = np.random.default_rng(n + light)
+    sites = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    sites = sites[np.sort(rng.permutation(125)[:n])]
+    typ = np.zeros(n, dtype=np.int32)
+    typ[rng.permutation(n)[:light]] = 1
+    a, b = 4.0 * 0.2 * 1.7 ** 12, 4.0 * 0.2 * 1.7 ** 6
+    s.update(pos=0.4 + 1.9 * sites + rng.uniform(-0.05, 0.05, (n, 3)), type=typ,
+             qscaled=water.SQRT_COULOMB * rng.uniform(-0.5, 0.5, n), mass=np.full(n, 16.0),
+             mol=np.arange(n, dtype=np.int32), excl=np.zeros((0, 3), dtype=np.int32), n=n)
+    s["lj"] = np.zeros((2, 2, 4))
+    s["lj"][0, 0] = a, b, a, b
+    return s
+
+
 CASES = {
     "one_water": lambda: _waters(1, (16.0, 16.0, 16.0)),
     "three_waters": lambda: _waters(3, (17.0, 19.0, 16.5)),
@@ -87,6 +107,9 @@ CASES = {
     "long_exclusion_lists": lambda: _merged(_waters(400, (20.0, 25.0, 24.0)), 4, False),
     "modified_pairs": lambda: _merged(_waters(399, (20.0, 25.0, 24.0)), 3, True),
     "flat": lambda: _waters(700, (60.0, 21.0, 16.0)),
+    "full_last_flush_104_37": lambda: _ball(104, 37),
+    "full_last_flush_99_5": lambda: _ball(99, 5),
+    "full_last_flush_104_95": lambda: _ball(104, 95),
 }
 
 
@@ -133,7 +156,7 @@ def test_fp64_against_oracle(name):
     assert pairs == O.restate_count_pairs(s, s["pos"])
 
 
-HVP_CASES = ["three_waters", "two_cutoffs", "odd_edges_unwrapped", "one_full_column",
+HVP_CASES = ["full_last_flush_104_37", "full_last_flush_104_95", "three_waters", "two_cutoffs", "odd_edges_unwrapped", "one_full_column",
              "long_exclusion_lists", "modified_pairs"]
 H = 1e-4
 
