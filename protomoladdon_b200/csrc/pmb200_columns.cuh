@@ -515,8 +515,10 @@ __device__ __forceinline__ int col_slot(int f0, int begin, unsigned runs, int &r
 // 1980), the Taylor polynomial to r^7 / 7! (|r| <= ln 2 / 2: 5e-9 left out), whose
 // last step rounds to nearest.  expf of the rounded square left nine tenths of
 // the Ewald energy's error (a bias of its last bit, and up to 4e-7 of the
-// exponential from the square's).  0 <= h < 80 (larger: any value).
+// exponential from the square's).  h >= 0; from 87 on e^{-87}, 1.6e-38, which no sum
+// here tells from zero (the exponent bits below would wrap).
 __device__ __forceinline__ float col_exp_neg(float h, float l) {
+  h = fminf(h, 87.0f);
   const float t = fmaf(-h, 1.44269504f, 12582912.0f);  // 1.5 2^23: rint in the low bits
   const float n = t - 12582912.0f;
   float r = fmaf(n, -0.693359375f, -h);

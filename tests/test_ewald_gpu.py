@@ -167,6 +167,20 @@ def test_seeded_boxes_vs_oracle(precision):
     assert np.abs(E.virial_matrix().ravel() - vo).max() <= tol * np.abs(vo).max()
 
 
+@pytest.mark.parametrize("accuracy", [1e-36, 1e-39, 1e-60, 1e-90])
+@pytest.mark.parametrize("form", ["poly5", "exact"])
+def test_accuracies_beyond_fp32s_exponents(form, accuracy):
+    """exp(-(alpha r)^2) below FP32's smallest number at the cutoff: such pairs add
+    nothing (the file's mixed bounds)."""
+    s = water.small_648()
+    alpha = np.sqrt(-np.log(accuracy)) / 8.0
+    fo, eo, vo, _ = O.restate_ewald_real(s, s["pos"], alpha, accuracy, form == "exact", 1)
+    F, E, (a, rc), _ = run(s, "mixed", form, alpha, accuracy, molvir=False)
+    assert rms_rel(F, fo) <= 1e-5
+    assert abs(E[0] - eo) <= 1e-6 * abs_pair_energy(s, a, rc)
+    assert np.abs(E.virial_matrix().ravel() - vo).max() <= 1e-5 * np.abs(vo).max()
+
+
 def test_large_box_mixed_against_fp64():
     """The 331,776-atom ion box at alpha 0.30, rc 12 (the large benchmark
     system): mixed against the FP64 kernel, and Newton's third law."""
