@@ -1039,9 +1039,11 @@ int launch_eval_clusters(pmb200_ctx *c, const double *d_pos, double *d_forces, d
   return PMB200_OK;
 }
 
+constexpr double kColMaxEdge = 160.0;  // box edge, in cutoffs (see col_prepare)
+
 // The column kernels' grid, neighbour columns, constants, tables and buffers
 // for the current box and topology (col_ok = false where they do not apply:
-// general cells and vacuum; the cell kernels then run).
+// general cells, vacuum and very long boxes; the cell kernels then run).
 int col_prepare(pmb200_ctx *c) {
   c->col_ok = false;
   if (!c->have_box || !c->have_topo) return PMB200_OK;
@@ -1049,6 +1051,13 @@ int col_prepare(pmb200_ctx *c) {
   const int n = c->n;
   const double rc = ctx_rc(c);
   const double *L = c->g.boxlen;
+  // a coordinate is held to 2^-32 of its edge.  Water in a box of growing length, RMS
+  // force error and Coulomb energy error per atom (kcal/mol) at rc 9: edges up to
+  // 300 A 7.7e-7, 2e-9; 1,200 A 7.7e-7, 8e-9; 2,400 A 8.2e-7, 2.3e-8; 19,200 A 3.0e-6,
+  // 1.6e-7; the cell kernels (coordinates within a cell) 9.5e-7 and 2e-8 to 6e-8
+  // throughout.  The FP64 kernels' box tests need edges below some 20,000 rc.
+  for (int a = 0; a < 3; a++)
+    if (L[a] > kColMaxEdge * rc) return PMB200_OK;
   ColGrid g{};
   // lengths in units of a power-of-two fraction of the x edge (about 4 A): one
   // quantum is then an exact FP32 number along x, and along y and z in cubes

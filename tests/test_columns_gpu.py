@@ -156,6 +156,27 @@ def test_fp64_against_oracle(name):
     assert pairs == O.restate_count_pairs(s, s["pos"])
 
 
+@pytest.mark.parametrize("precision,length,tol", [
+    ("mixed", 1279.0, 2e-6), ("mixed", 1281.0, 2e-6), ("mixed", 19200.0, 2e-6),
+    ("fp64", 1281.0, 1e-12), ("fp64", 6e5, 1e-12)])
+def test_long_boxes(precision, length, tol):
+    """The column kernels hold a coordinate to 2^-32 of its edge (at 19,200 A three
+    times the FP32 force error of about 1e-6): longer boxes run on the cell kernels,
+    with the same errors as short ones."""
+    s = _waters(400, (20.0, 20.0, length), (20.0, 20.0, 30.0), rc=8.0)
+    s["pos"] = s["pos"] + np.array([0.0, 0.0, 0.37 * length])
+    f = NonbondedCutoffB200SystemForce(s["ron"], s["rc_lj"], s["rc_coul"], s["rc_alg"],
+                                       precision=precision)
+    F, E = np.zeros_like(s["pos"]), ScalarStructure()
+    f.evaluate(PeriodicTopology.from_dict(s), s["pos"], F, E)
+    pairs = f.last_pair_count()
+    f.close()
+    fo, eo, _, _ = O.restate_eval(s, s["pos"], virial_mode=0)
+    assert np.sqrt(((F - fo) ** 2).sum()) <= tol * np.sqrt((fo ** 2).sum())
+    assert max(abs(E[0] - eo[0]), abs(E[1] - eo[1])) <= tol * 100.0 * s["n"]
+    assert abs(pairs - O.restate_count_pairs(s, s["pos"])) <= (precision == "mixed")
+
+
 HVP_CASES = ["full_last_flush_104_37", "full_last_flush_104_95", "three_waters", "two_cutoffs", "odd_edges_unwrapped", "one_full_column",
              "long_exclusion_lists", "modified_pairs"]
 H = 1e-4
