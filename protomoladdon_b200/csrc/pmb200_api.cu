@@ -89,6 +89,7 @@ struct pmb200_ctx {
   int col_clusters = 0;       // upper bound of the clusters
   char *d_carena = nullptr;   // the column kernels' buffers and tables
   size_t carena_bytes = 0, col_ncol_alloc = 0;
+  int col_tables = 0;         // which copy of the tables is in use (col_prepare)
   bool col_count_zero = false;
   double *d_csq = nullptr;
   // FP64 kernels: wrapped positions (caller and slot order), a direction
@@ -1126,7 +1127,7 @@ int col_prepare(pmb200_ctx *c) {
   c->cg = g;
   // buffers: the cell kernels' where they are large enough, the rest carved from
   // one allocation (a batch's hundreds of contexts would otherwise spend their
-  // construction in the allocator); the tables last, back to back for one upload
+  // construction in the allocator)
   const bool room = (size_t)g.nslot <= c->slot_room;
   const bool rows = (long long)c->col_clusters * g.nparts <=
                     (long long)c->ncell_alloc * kMaxCellSlots;
@@ -1136,14 +1137,29 @@ int col_prepare(pmb200_ctx *c) {
   c->d_cspos64 = c->d_spos64;
   c->d_cw = reinterpret_cast<double4 *>(c->d_rel_lo);
   c->d_cpartial = c->d_partial;
+  // The tables come first, in kTables copies used in turn: an evaluation queued
+  // before this call still reads its own (its other arrays are next written by
+  // work that follows it on its stream).  After the last copy the arena is
+  // allocated anew, and freeing the old one waits for what runs on it.
+  constexpr int kTables = 16;
   const size_t t2 = (size_t)c->ntypes * c->ntypes;
-  auto carve = [&](char *base) {
+  const int copies = t2 > 256 ? 1 : kTables;
+  auto carve = [&](char *base, int copy) {
     size_t off = 0;
     auto take = [&](auto *&p, size_t count) {
       using T = std::remove_pointer_t<std::remove_reference_t<decltype(p)>>;
       if (base) p = reinterpret_cast<T *>(base + off);
       off = (off + sizeof(T) * count + 255) & ~(size_t)255;
     };
+    for (int k = 0; k < copies; k++) {
+      char *const b = base;
+      if (k != copy) base = nullptr;
+      take(c->d_ljc64, 2 * t2);
+      take(c->d_ljc32, t2);
+      take(c->d_ljact, (size_t)c->ntypes);
+      take(c->d_cst, (size_t)kColMaxCls);
+      base = b;
+    }
     take(c->d_cctl, 4);
     if (!room) {
       take(c->d_cspos, (size_t)g.nslot);
@@ -1157,19 +1173,17 @@ int col_prepare(pmb200_ctx *c) {
     take(c->d_zs, (size_t)g.ncol * (g.nsz + 1));
     if (!rows) take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
     take(c->d_icom, (size_t)std::max(c->nmol, 1));
-    take(c->d_ljc64, 2 * t2);
-    take(c->d_ljc32, t2);
-    take(c->d_ljact, (size_t)c->ntypes);
-    take(c->d_cst, (size_t)kColMaxCls);
     return off;
   };
-  const size_t want = carve(nullptr);
-  if (want > c->carena_bytes) {
+  const size_t want = carve(nullptr, 0);
+  if (want > c->carena_bytes || ++c->col_tables >= copies) {
+    const size_t bytes = std::max(want, c->carena_bytes);
     c->carena_bytes = 0;
-    CK(dalloc(c->d_carena, want));
-    c->carena_bytes = want;
+    CK(dalloc(c->d_carena, bytes));
+    c->carena_bytes = bytes;
+    c->col_tables = 0;
   }
-  carve(c->d_carena);
+  carve(c->d_carena, c->col_tables);
   // (the counts keep their place: every evaluation leaves them zero)
   if (c->col_ncol_alloc < (size_t)g.ncol) {
     c->col_ncol_alloc = 0;

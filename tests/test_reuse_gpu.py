@@ -71,3 +71,39 @@ def test_one_context_across_grids():
         # the two paths (energy and forces-only launches) agree to rounding
         assert np.sqrt(((Fh - Fd) ** 2).sum() / (Fd ** 2).sum()) <= 1e-6, k
     reused.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_new_boxes_while_evaluations_are_queued(precision):
+    """A box set while earlier evaluations have still to run leaves them theirs:
+    only the height changes, and with it the column grid.  Bit for bit the forces
+    of contexts of their own."""
+    s = water.water_box(14, rc=8.0, ron=7.0, seed=5)
+    boxes = [dict(s, box=s["box"] * np.array([1.0, 1.0, 1.0 + 0.05 * (k % 7)]))
+             for k in range(40)]
+    make = lambda: NonbondedCutoffB200SystemForce(s["ron"], s["rc_lj"], s["rc_coul"],  # noqa: E731
+                                                  s["rc_alg"], precision=precision)
+    pos = torch.tensor(s["pos"], dtype=torch.float64, device="cuda")
+    want = []
+    for b in boxes[:7]:
+        f = make()
+        frc = torch.zeros_like(pos)
+        f.evaluate_device(PeriodicTopology.from_dict(b), pos.data_ptr(), frc.data_ptr(), None, 0, 1)
+        torch.cuda.synchronize()
+        f.close()
+        want.append(frc)
+    topo = PeriodicTopology.from_dict(s)
+    f = make()
+    f.number_of_blocks(topo)
+    frc = [torch.zeros_like(pos) for _ in boxes]
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for k, (b, r) in enumerate(zip(boxes, frc)):
+        topo.e = np.diag(b["box"])
+        for _ in range(1 if k else 50):  # (work ahead of the others)
+            f.evaluate_device(topo, pos.data_ptr(), r.data_ptr(), None, 0, st.cuda_stream)
+    st.synchronize()
+    f.sync()
+    f.close()
+    for k, r in enumerate(frc[1:], 1):
+        assert torch.equal(r, want[k % 7]), k
