@@ -1041,6 +1041,7 @@ int launch_eval_clusters(pmb200_ctx *c, const double *d_pos, double *d_forces, d
 }
 
 constexpr double kColMaxEdge = 160.0;  // box edge, in cutoffs (see col_prepare)
+constexpr double kColMaxSide = 0.7;    // column width, in cutoffs
 
 // The column kernels' grid, neighbour columns, constants, tables and buffers
 // for the current box and topology (col_ok = false where they do not apply:
@@ -1072,13 +1073,18 @@ int col_prepare(pmb200_ctx *c) {
     g.q[a] = (float)g.qd[a];
   }
   // columns about the edge of a cube of kColI atoms wide (measured on water:
-  // 0.9 to 1.15 times that edge within 2%), slabs 0.3 of it high
+  // 0.9 to 1.15 times that edge within 2%), slabs 0.3 of it high.  At most
+  // kColMaxSide cutoffs, since the mean density says little of a box that is not
+  // uniformly filled: 41k atoms of water in a cube of 3, 4 and 6 times their edge
+  // take 88, 88 and 119 us (forces) so, 106, 106 and 135 with one cutoff, 137, 185 and
+  // 201 with 1.4; filled 90.  A gas of 1/216 of water's density, 41k atoms, takes 45,
+  // 41 and 35 us.
   const double rlist = rc * (1.0 + 1e-5);
-  double side = std::cbrt(kColI * L[0] * L[1] * L[2] / n);
+  double side = std::min(std::cbrt(kColI * L[0] * L[1] * L[2] / n), kColMaxSide * rc);
   for (;; side *= 1.25) {
     g.ncx = std::max(1, std::min(16384, (int)std::lround(L[0] / side)));
     g.ncy = std::max(1, std::min(16384, (int)std::lround(L[1] / side)));
-    if ((long long)g.ncx * g.ncy > (1 << 22)) continue;
+    if ((long long)g.ncx * g.ncy > std::max(256, n)) continue;
     const double w[2] = {L[0] / g.ncx, L[1] / g.ncy};
     // neighbour classes (offsets modulo the grid) by the gap between columns
     std::vector<std::pair<double, short2>> cls;
@@ -1112,13 +1118,16 @@ int col_prepare(pmb200_ctx *c) {
   }
   g.ncol = g.ncx * g.ncy;
   g.nsz = std::max(1, std::min(kColMaxSlabs, (int)std::lround(L[2] / (0.3 * side))));
-  g.cap = (int)std::min<long long>(n, 2LL * n / g.ncol + 64);
+  // buckets of 32 times the mean column, 128 bytes an atom: an unevenly filled box
+  // has long columns (41k atoms of water in three times their edge 12 times the mean;
+  // with twice the mean the sort took 800 us there, 7 in the full box)
+  g.cap = (int)std::min<long long>(n, std::max(2LL * n / g.ncol + 64, 32LL * n / g.ncol));
   g.inv_hs = (float)(g.nsz * u / L[2]);
   g.rc2 = (float)(rlist * rlist / (u * u));
   g.inv_unit = 1.0 / u;
   for (int a = 0; a < 3; a++) g.hmax[a] = (float)((0.5 * L[a] - rlist) / u - 1e-3);
   g.qscale = (float)(1.0 / std::sqrt(u));
-  const long long slots = (long long)n + (long long)(kColI - 1) * g.ncol;
+  const long long slots = (long long)n + (long long)(kColI - 1) * std::min(n, g.ncol);
   g.nslot = (int)((slots + kColI - 1) / kColI * kColI);
   c->col_clusters = g.nslot / kColI;
   const int cl = n / kColI;
@@ -3804,7 +3813,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
     y.col0 = (int)col_sys.size();
     y.slot0 = (int)slots;
     y.zs0 = (int)zs;
-    y.bucket0 = (int)bucket;
+    y.bucket0 = bucket;
     y.st0 = (int)cls.size();
     y.lj0 = (int)l32.size();
     y.act0 = (int)act.size();
@@ -3820,7 +3829,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
       b->col_parts.back() = c->cg.nparts;
       b->col_full = b->col_full && c->col_full;
       b->col_mod = b->col_mod || c->has_modified;
-      b->col_small = b->col_small && c->cg.cap <= kColSortCapS && c->cg.ncol <= 1024;
+      b->col_small = b->col_small && 2LL * c->n / c->cg.ncol + 64 <= kColSortCapS && c->cg.ncol <= 1024;
       const size_t t2 = (size_t)c->ntypes * c->ntypes;
       l32.resize(l32.size() + t2);
       l64.resize(l64.size() + 2 * t2);
@@ -3834,7 +3843,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
     }
     b->h_col.push_back(y);
   }
-  if (slots > (1LL << 30) || zs > (1LL << 30) || bucket > (1LL << 30)) {
+  if (slots > (1LL << 30) || zs > (1LL << 30)) {
     b->col = false;  // (the cell kernels take it)
     return PMB200_OK;
   }

@@ -156,18 +156,18 @@ static __global__ void k_col_index(int n, const double *__restrict__ pos, ColGri
 
 // One column's sort by one block: base is its first slot, rank0 its first rank.  Order: slab, height,
 // atom index (the layout, and every sum over it, is the same on every run).
-// A counting sort by slab in shared memory, then ranks among the two or three
-// atoms of a slab; the slabs' first slots come with it.  (Ranks counted against
-// the whole column took 50 us on the 327k-atom box.)  A column of more than cap
-// atoms, whose bucket is incomplete, collects them from the whole list i0 ..
-// i0 + n - 1; one that exceeds the shared buffer works from global memory
-// (scratch: its own slots of a slot-sized list).
+// A counting sort by slab, then ranks among the few atoms of a slab; the slabs'
+// first slots come with it.  (Ranks counted against the whole column took 50 us
+// on the 327k-atom box.)  In shared memory where the column fits, else through
+// the column's slots of a slot-sized list in global memory (scratch).  A column of
+// more than cap atoms, whose bucket is incomplete, finds them in the whole list
+// i0 .. i0 + n - 1, which it reads twice.
 template <int kCap>
 struct ColSortSmem {
   unsigned long long key[kCap];
   int list[kCap];
   int first[kColMaxSlabs + 1];
-  int warp[8], n;
+  int warp[8];
 };
 template <int kThreads, int kCap>
 __device__ __forceinline__ void col_sort_column(
@@ -192,41 +192,56 @@ __device__ __forceinline__ void col_sort_column(
     if (sw)
       sw[base + rank] = make_double4(w[3 * (size_t)i], w[3 * (size_t)i + 1], w[3 * (size_t)i + 2], 0.0);
   };
+  // the column's atoms: from its bucket, or from the whole list
+  const bool whole = cnt > g.cap, shared = !whole && cnt <= kCap;
+  auto each = [&](auto &&f) {
+    if (!whole) {
+      for (int k = t; k < cnt; k += T) {
+        const int i = bucket[k];
+        f(k, i, (unsigned)ipos[i].z);
+      }
+    } else {
+#pragma unroll 4
+      for (int k = t; k < n; k += T) {
+        const int4 p = ipos[i0 + k];
+        if (col_of(g, (unsigned)p.x, (unsigned)p.y) == col) f(k, i0 + k, (unsigned)p.z);
+      }
+    }
+  };
   for (int k = t; k < g.nsz; k += T) sm.first[k] = 0;
   __syncthreads();
-  if (cnt <= g.cap && cnt <= kCap) {
-    for (int k = t; k < cnt; k += T) {
-      const int i = bucket[k];
-      const unsigned z = (unsigned)ipos[i].z;
-      sm.key[k] = ((unsigned long long)z << 32) | (unsigned)i;
-      atomicAdd(&sm.first[__umulhi(z, nsz)], 1);
-    }
-    __syncthreads();
-    // slab counts -> first entries (exclusive), a warp-sized piece at a time
-    for (int c0 = 0, carry = 0; c0 < g.nsz; c0 += T) {
-      const int v = c0 + t < g.nsz ? sm.first[c0 + t] : 0;
-      int incl = v;
+  each([&](int k, int i, unsigned z) {
+    if (shared) sm.key[k] = ((unsigned long long)z << 32) | (unsigned)i;
+    atomicAdd(&sm.first[__umulhi(z, nsz)], 1);
+  });
+  __syncthreads();
+  // slab counts -> first entries (exclusive), a block-sized piece at a time
+  for (int c0 = 0, carry = 0; c0 < g.nsz; c0 += T) {
+    const int v = c0 + t < g.nsz ? sm.first[c0 + t] : 0;
+    int incl = v;
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += u;
-      }
-      if (lane == 31) sm.warp[wp] = incl;
-      __syncthreads();
-      int before = carry, total = 0;
-      for (int w = 0; w < T / 32; w++) {
-        if (w < wp) before += sm.warp[w];
-        total += sm.warp[w];
-      }
-      if (c0 + t < g.nsz) {
-        sm.first[c0 + t] = before + incl - v;
-        zs[c0 + t] = base + before + incl - v;
-      }
-      carry += total;
-      __syncthreads();
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += u;
     }
-    if (t == 0) zs[g.nsz] = base + cnt;
-    // scattered to their slabs in any order (first then holds each slab's end)
+    if (lane == 31) sm.warp[wp] = incl;
+    __syncthreads();
+    int before = carry, total = 0;
+    for (int w = 0; w < T / 32; w++) {
+      if (w < wp) before += sm.warp[w];
+      total += sm.warp[w];
+    }
+    if (c0 + t < g.nsz) {
+      sm.first[c0 + t] = before + incl - v;
+      zs[c0 + t] = base + before + incl - v;
+    }
+    carry += total;
+    __syncthreads();
+  }
+  if (t == 0) zs[g.nsz] = base + cnt;
+  // scattered to their slabs in any order (first then holds each slab's end), then
+  // ranked among the slab's atoms
+  if (shared) {
     for (int k = t; k < cnt; k += T)
       sm.list[atomicAdd(&sm.first[__umulhi((unsigned)(sm.key[k] >> 32), nsz)], 1)] = k;
     __syncthreads();
@@ -240,36 +255,23 @@ __device__ __forceinline__ void col_sort_column(
       put(i, rank, ipos[i]);
     }
   } else {
-    if (cnt > g.cap) {
-      if (t == 0) sm.n = 0;
-      __syncthreads();
-      for (int k = t; k < n; k += T) {
-        const int4 p = ipos[i0 + k];
-        if (col_of(g, (unsigned)p.x, (unsigned)p.y) == col)
-          scratch[base + atomicAdd(&sm.n, 1)] = i0 + k;
-      }
-    } else {
-      for (int k = t; k < cnt; k += T) scratch[base + k] = bucket[k];
-    }
+    int *list = scratch + base;
+    each([&](int, int i, unsigned z) { list[atomicAdd(&sm.first[__umulhi(z, nsz)], 1)] = i; });
     __syncthreads();
-    for (int k = t; k < cnt; k += T) {
-      const int i = scratch[base + k];
+    for (int e = t; e < cnt; e += T) {
+      const int i = list[e];
       const int4 p = ipos[i];
-      int rank = 0;
-      for (int m = 0; m < cnt; m++) {
-        const int o = scratch[base + m];
+      const unsigned z = (unsigned)p.z;
+      const int s = (int)__umulhi(z, nsz);
+      const int lo = s ? sm.first[s - 1] : 0, hi = sm.first[s];
+      int rank = lo;
+      for (int m = lo; m < hi; m++) {
+        const int o = list[m];
         const unsigned zo = (unsigned)ipos[o].z;
-        rank += zo < (unsigned)p.z || (zo == (unsigned)p.z && o < i);
+        rank += zo < z || (zo == z && o < i);
       }
       put(i, rank, p);
     }
-    __syncthreads();
-    // atom k opens the slabs above the previous atom's up to its own
-    auto slab = [&](int k) -> int {
-      return k < 0 ? -1 : (k >= cnt ? g.nsz : (int)__umulhi((unsigned)spos[base + k].z, nsz));
-    };
-    for (int k = t; k <= cnt; k += T)
-      for (int s = slab(k - 1) + 1; s <= slab(k); s++) zs[s] = base + k;
   }
   const int end = (cnt + kColI - 1) / kColI * kColI;
   for (int k = cnt + t; k < end; k += T) {
@@ -1215,7 +1217,8 @@ struct ColBatchSys {
   ColGrid g;
   MixedConsts mc;
   double fscale;            // fixed point -> force: 2^-32 / unit
-  int atom0, natoms, col0, slot0, zs0, bucket0;
+  int atom0, natoms, col0, slot0, zs0;
+  long long bucket0;
   int st0, st_n;            // neighbour-column classes
   int lj0, act0, ntypes;    // LJ tables (float4; double2 at 2 lj0), LJ-active flags
 };
@@ -1242,8 +1245,8 @@ static __global__ void k_col_index_batch(int N, const double *__restrict__ pos,
 
 // One block per column of the batch; col_sys: its system.  ctl[s]: clusters.
 // Bound by each block's chain of loads and barriers; what helps is blocks in
-// flight.  Where no system's buckets hold more than kColSortCapS atoms (columns
-// beyond a bucket never use the shared buffer) blocks take kColSortThreadsS threads
+// flight.  Where twice every system's mean column and 64 fit kColSortCapS atoms
+// (longer ones go through global memory) blocks take kColSortThreadsS threads
 // and 9 KB instead of 22 KB: an evaluation of 512 boxes of 300 to 6,000 atoms
 // 2,208 -> 2,172 us (32 and 64 threads the same within 5).
 template <int kThreads, int kCap>

@@ -1,7 +1,7 @@
 """The column kernels (the evaluation path of orthogonal periodic boxes) at the
 shapes where their layout has edges: clusters of 8 atoms and blocks of 32 staged
 ones that do not fill, boxes of exactly two cutoffs, columns that are their own
-opposite, columns whose atoms overflow their bucket or the sort's shared memory,
+opposite, columns whose atoms overflow their bucket, the sort's shared memory or both,
 clusters taller than the cutoff, exclusion lists longer than a warp, a buffer that
 is nearly full at the end -- against the FP64 oracle.
 
@@ -107,6 +107,8 @@ CASES = {
     "long_exclusion_lists": lambda: _merged(_waters(400, (20.0, 25.0, 24.0)), 4, False),
     "modified_pairs": lambda: _merged(_waters(399, (20.0, 25.0, 24.0)), 3, True),
     "flat": lambda: _waters(700, (60.0, 21.0, 16.0)),
+    "tall_block_in_vacuum": lambda: _waters(727, (150.0, 140.0, 400.0), (11.0, 11.0, 180.0)),
+    "thread_in_vacuum": lambda: _waters(1540, (52.5, 52.5, 1250.0), (6.2, 6.2, 1197.0), rc=11.0),
     "full_last_flush_104_37": lambda: _ball(104, 37),
     "full_last_flush_99_5": lambda: _ball(99, 5),
     "full_last_flush_104_95": lambda: _ball(104, 95),
