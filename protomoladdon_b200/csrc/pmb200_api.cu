@@ -97,6 +97,7 @@ struct pmb200_ctx {
   int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr, *d_icom = nullptr;
   int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_cscratch = nullptr;
   int *d_cctl = nullptr;
+  int2 *d_csums = nullptr;    // k_col_scan's (kColScan columns or more)
   unsigned char *d_ljact = nullptr;
   float4 *d_ljc32 = nullptr;
   double2 *d_ljc64 = nullptr;
@@ -1180,6 +1181,7 @@ int col_prepare(pmb200_ctx *c) {
     take(c->d_csq, (size_t)g.nslot);
     take(c->d_bucket, (size_t)g.ncol * g.cap);
     take(c->d_zs, (size_t)g.ncol * (g.nsz + 1));
+    take(c->d_csums, g.ncol >= kColScan ? (size_t)g.ncol : 0);
     if (!rows) take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
     take(c->d_icom, (size_t)std::max(c->nmol, 1));
     return off;
@@ -1241,13 +1243,17 @@ int launch_col_build(pmb200_ctx *c, const double *d_pos, cudaStream_t st,
            (unsigned)((n + 255) / 256 + (mols.n + 255) / 256), 256, 0, st, false, n, d_pos, g,
            (const double *)c->d_q, c->d_ipos, c->d_ccount, c->d_bucket, clear,
            clear ? nclear : 0, c->d_err, fp64 ? c->d_dpos : nullptr, mols);
+  const bool scan = g.ncol >= kColScan;
+  if (scan)
+    launch_k(k_col_scan, 1, 1024, 0, st, true, g.ncol, (const int *)c->d_ccount, c->d_csums);
   launch_k(k_col_sort, (unsigned)g.ncol, kColSortThreads, 0, st, true, n, g,
            (const int4 *)c->d_ipos, (const int *)c->d_ccount, (const int *)c->d_bucket,
            (const int *)c->d_type, (const int *)c->d_mol, (const unsigned char *)c->d_ljact,
            (const double *)c->d_q, c->d_cspos, c->d_csmeta, c->d_csq, c->d_sidx, c->d_zs,
            c->d_cscratch,
            c->d_cctl, fp64 ? (const double4 *)c->d_dpos : (const double4 *)nullptr,
-           fp64 ? c->d_cspos64 : (double4 *)nullptr, d_w, d_w ? c->d_cw : (double4 *)nullptr);
+           fp64 ? c->d_cspos64 : (double4 *)nullptr, d_w, d_w ? c->d_cw : (double4 *)nullptr,
+           scan ? (const int2 *)c->d_csums : (const int2 *)nullptr);
   CK(cudaGetLastError());
   return PMB200_OK;
 }
@@ -3571,6 +3577,7 @@ struct pmb200_batch {
   ColBatchSys *d_col = nullptr;
   int *d_ccount = nullptr, *d_bucket = nullptr, *d_zs = nullptr, *d_scratch = nullptr;
   int *d_ctl = nullptr, *d_col_sys = nullptr;
+  int2 *d_sums = nullptr;       // k_col_scan's, where a system has kColScan columns
   int4 *d_ipos = nullptr, *d_cspos = nullptr, *d_csmeta = nullptr;
   double *d_csq = nullptr;
   short2 *d_cst = nullptr;
@@ -3732,11 +3739,12 @@ int batch_launch_eval(pmb200_batch *b, const double *d_pos, double *d_forces, do
     k_col_index_batch<<<(N + 255) / 256, 256, 0, st>>>(N, d_pos, b->d_col, b->d_atom_sys, b->d_q,
                                                        b->d_ipos, b->d_ccount, b->d_bucket,
                                                        b->d_facc, b->d_err);
+    if (b->d_sums) k_col_scan<<<1, 1024, 0, st>>>(b->ncol, b->d_ccount, b->d_sums);
     auto sort = [&](auto kernel, int threads) {
       kernel<<<b->ncol, threads, 0, st>>>(
           b->d_col, b->d_col_sys, b->d_ipos, b->d_ccount, b->d_bucket, b->d_type, b->d_mol,
           b->d_ljact, b->d_q, b->d_cspos, b->d_csmeta, b->d_csq, b->d_sidx, b->d_zs,
-          b->d_scratch, b->d_ctl);
+          b->d_scratch, b->d_ctl, b->d_sums);
     };
     if (b->col_small) sort(k_col_sort_batch<kColSortThreadsS, kColSortCapS>, kColSortThreadsS);
     else sort(k_col_sort_batch<kColSortThreads, kColSortCap>, kColSortThreads);
@@ -3805,6 +3813,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
   std::vector<double2> l64;
   std::vector<unsigned char> act;
   long long slots = 0, zs = 0, bucket = 0;
+  bool scan = false;
   for (int s = 0; s < b->nsys; s++) {
     pmb200_ctx *c = systems[s];
     ColBatchSys y{};
@@ -3827,6 +3836,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
       cls.insert(cls.end(), c->cst.off, c->cst.off + c->cst.n);
       col_sys.insert(col_sys.end(), c->cg.ncol, s);
       b->col_parts.back() = c->cg.nparts;
+      scan = scan || c->cg.ncol >= kColScan;
       b->col_full = b->col_full && c->col_full;
       b->col_mod = b->col_mod || c->has_modified;
       b->col_small = b->col_small && 2LL * c->n / c->cg.ncol + 64 <= kColSortCapS && c->cg.ncol <= 1024;
@@ -3857,6 +3867,7 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
   BCK(dalloc(b->d_scratch, S));
   BCK(dalloc(b->d_ctl, (size_t)b->nsys));
   BCK(cudaMemset(b->d_ctl, 0, sizeof(int) * (size_t)b->nsys));
+  if (scan) BCK(dalloc(b->d_sums, col_sys.size()));
   BCK(dalloc(b->d_col_sys, col_sys.size()));
   BCK(dalloc(b->d_ipos, N));
   BCK(dalloc(b->d_cspos, S));
@@ -3893,7 +3904,7 @@ int pmb200_batch_destroy(pmb200_batch *b) {
   dfree(b->d_partial); dfree(b->d_pairs); dfree(b->d_scratch_f); dfree(b->d_tasks);
   dfree(b->d_rows_start); dfree(b->d_rows);
   dfree(b->d_col); dfree(b->d_ccount); dfree(b->d_bucket); dfree(b->d_zs); dfree(b->d_scratch);
-  dfree(b->d_ctl); dfree(b->d_col_sys); dfree(b->d_ipos); dfree(b->d_cspos); dfree(b->d_csmeta);
+  dfree(b->d_ctl); dfree(b->d_sums); dfree(b->d_col_sys); dfree(b->d_ipos); dfree(b->d_cspos); dfree(b->d_csmeta);
   dfree(b->d_csq); dfree(b->d_cst); dfree(b->d_ljact); dfree(b->d_ljc32); dfree(b->d_ljc64);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);

@@ -41,6 +41,7 @@ constexpr int kColMaxCls = 256;   // neighbour-column classes
 constexpr int kColSortCap = 1536; // atoms a column sort holds in shared memory,
 constexpr int kColSortCapS = 384; // and in a batch of small boxes (k_col_sort_batch)
 constexpr int kColMaxSlabs = 1024;
+constexpr int kColScan = 12000;   // columns from which on k_col_scan sums the counts
 constexpr int kColSortThreads = 256, kColSortThreadsS = 128;
 
 struct ColGrid {
@@ -280,9 +281,8 @@ __device__ __forceinline__ void col_sort_column(
   }
 }
 
-// The clusters and atoms of the columns before `col` (each block sums them
-// itself: a few thousand counts at most on the sizes a GPU holds, and no scan
-// launch).
+// The clusters and atoms of the columns before `col`: each block of the sort sums
+// them itself where the counts are few, else k_col_scan has (kColScan).
 template <int kThreads, int kCap>
 __device__ __forceinline__ void col_before(const int *__restrict__ count, int col, int &clusters,
                                            int &atoms, ColSortSmem<kCap> &sm) {
@@ -309,7 +309,62 @@ __device__ __forceinline__ void col_before(const int *__restrict__ count, int co
   }
 }
 
-// One block per column.  ctl[0]: the number of clusters.
+// Exclusive prefix sums {clusters, atoms} over all columns, one block of 1024
+// threads, four columns a thread and round.  The blocks' own sums are quadratic in
+// the columns: forces of water films 20 A thick (8,464 / 16,900 / 26,244 / 126,736
+// columns) 461 / 918 / 1,427 / 8,127 us, with this launch 463 / 909 / 1,392 /
+// 6,680.
+static __global__ void __launch_bounds__(1024)
+k_col_scan(int ncol, const int *__restrict__ count, int2 *__restrict__ before) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ int2 sh[32];
+  const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+  int2 carry = make_int2(0, 0);
+  for (int c0 = 0; c0 < ncol; c0 += 4096) {
+    const int c = c0 + 4 * t;
+    int v[4];
+    int2 sum = make_int2(0, 0);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      v[k] = c + k < ncol ? count[c + k] : 0;
+      sum.x += (v[k] + kColI - 1) / kColI;
+      sum.y += v[k];
+    }
+    int2 incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl.x, off);
+      const int y = __shfl_up_sync(0xffffffffu, incl.y, off);
+      if (lane >= off) {
+        incl.x += x;
+        incl.y += y;
+      }
+    }
+    if (lane == 31) sh[wp] = incl;
+    __syncthreads();
+    int2 at = make_int2(carry.x + incl.x - sum.x, carry.y + incl.y - sum.y);
+#pragma unroll 8
+    for (int w = 0; w < 32; w++) {
+      const int2 s = sh[w];
+      if (w < wp) {
+        at.x += s.x;
+        at.y += s.y;
+      }
+      carry.x += s.x;
+      carry.y += s.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (c + k < ncol) before[c + k] = at;
+      at.x += (v[k] + kColI - 1) / kColI;
+      at.y += v[k];
+    }
+    __syncthreads();
+  }
+}
+
+// One block per column.  ctl[0]: the number of clusters.  sums: k_col_scan's, or null.
 static __global__ void __launch_bounds__(kColSortThreads)
 k_col_sort(int n, ColGrid g, const int4 *__restrict__ ipos, const int *__restrict__ count,
            const int *__restrict__ bucket, const int *__restrict__ type,
@@ -318,13 +373,18 @@ k_col_sort(int n, ColGrid g, const int4 *__restrict__ ipos, const int *__restric
            double *__restrict__ sq, int *__restrict__ sidx, int *__restrict__ zs,
            int *__restrict__ scratch, int *__restrict__ ctl, const double4 *__restrict__ dpos,
            double4 *__restrict__ spos64, const double *__restrict__ w,
-           double4 *__restrict__ sw) {
+           double4 *__restrict__ sw, const int2 *__restrict__ sums) {
   pdl_trigger();
   pdl_wait();
   __shared__ ColSortSmem<kColSortCap> sm;
   const int col = blockIdx.x, t = threadIdx.x;
   int before, atoms;
-  col_before<kColSortThreads>(count, col, before, atoms, sm);
+  if (sums) {
+    before = sums[col].x;
+    atoms = sums[col].y;
+  } else {
+    col_before<kColSortThreads>(count, col, before, atoms, sm);
+  }
   const int cnt = count[col];
   if (col == g.ncol - 1 && t == 0) ctl[0] = before + (cnt + kColI - 1) / kColI;
   __syncthreads();
@@ -1257,13 +1317,20 @@ k_col_sort_batch(const ColBatchSys *__restrict__ sys, const int *__restrict__ co
                  const int *__restrict__ mol, const unsigned char *__restrict__ ljact,
                  const double *__restrict__ q, int4 *__restrict__ spos,
                  int4 *__restrict__ smeta, double *__restrict__ sq, int *__restrict__ sidx,
-                 int *__restrict__ zs, int *__restrict__ scratch, int *__restrict__ ctl) {
+                 int *__restrict__ zs, int *__restrict__ scratch, int *__restrict__ ctl,
+                 const int2 *__restrict__ sums) {
   __shared__ ColSortSmem<kCap> sm;
   const int s = col_sys[blockIdx.x], t = threadIdx.x;
   const ColBatchSys &b = sys[s];
   const int col = (int)blockIdx.x - b.col0;
   int before, atoms;
-  col_before<kThreads>(count + b.col0, col, before, atoms, sm);
+  if (sums) {  // (over all systems)
+    const int2 first = sums[b.col0], here = sums[blockIdx.x];
+    before = here.x - first.x;
+    atoms = here.y - first.y;
+  } else {
+    col_before<kThreads>(count + b.col0, col, before, atoms, sm);
+  }
   const int cnt = count[blockIdx.x];
   if (col == b.g.ncol - 1 && t == 0) ctl[s] = before + (cnt + kColI - 1) / kColI;
   __syncthreads();
