@@ -3853,7 +3853,8 @@ int batch_create_columns(pmb200_batch *b, pmb200_ctx *const *systems) {
     }
     b->h_col.push_back(y);
   }
-  if (slots > (1LL << 30) || zs > (1LL << 30)) {
+  // (staged entries hold a force's offset, 8 bytes times its atom's rank, in 32 bits)
+  if (b->N > (1 << 29) || slots > (1LL << 30) || zs > (1LL << 30)) {
     b->col = false;  // (the cell kernels take it)
     return PMB200_OK;
   }
