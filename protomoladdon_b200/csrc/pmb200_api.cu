@@ -117,6 +117,8 @@ struct pmb200_ctx {
   bool have_topo = false, have_box = false, have_mass = false;
   double csf = 1.0;
   std::vector<double> h_lj;  // ntypes^2 * 4
+  std::vector<int> h_ex_start;  // the exclusion lists of d_ex_start and d_ex (batches)
+  std::vector<int2> h_ex;
   int *d_type = nullptr, *d_mol = nullptr;
   double *d_q = nullptr, *d_mass = nullptr;
   int *d_ex_start = nullptr;
@@ -140,7 +142,8 @@ struct pmb200_ctx {
   int *d_cell_of = nullptr, *d_slot = nullptr, *d_tmp = nullptr, *d_sidx = nullptr;
   float4 *d_rel32 = nullptr, *d_spos32 = nullptr;
   float4 *d_rel_lo = nullptr, *d_spos_lo = nullptr;  // FP32 coordinate residuals (one allocation)
-  size_t slot_room = 0;  // slots that d_spos32, d_spos64 and (as double4) d_rel_lo hold
+  // slots that d_tmp, d_spos32, d_spos64, d_smeta, d_cblo and (as double4) d_rel_lo hold
+  size_t slot_room = 0;
   double4 *d_rel64 = nullptr, *d_spos64 = nullptr;
   int2 *d_smeta = nullptr;
   // force accumulator, sorted order: [3][n] 2^-32 quanta (mixed) or [6][n]
@@ -503,22 +506,22 @@ int ensure_atom_buffers(pmb200_ctx *c) {
   const size_t n = (size_t)std::max(c->n, 1);
   CK(dalloc(c->d_cell_of, n));
   CK(dalloc(c->d_slot, n));
-  CK(dalloc(c->d_tmp, n));
-  CK(dalloc(c->d_sidx, n));
   // (with room for the column kernels' slots, which share some of them: an
   // evaluation runs on one kind of kernel)
   const size_t slots = n + n / 4 + 64;
   c->slot_room = 0;
+  CK(dalloc(c->d_tmp, slots));
+  CK(dalloc(c->d_sidx, n));
   CK(dalloc(c->d_rel32, n));
   CK(dalloc(c->d_spos32, slots));
   CK(dalloc(c->d_rel_lo, 2 * slots));
   c->d_spos_lo = c->d_rel_lo + slots;
   CK(dalloc(c->d_rel64, n));
   CK(dalloc(c->d_spos64, slots));
-  c->slot_room = slots;
-  CK(dalloc(c->d_smeta, n));
+  CK(dalloc(c->d_smeta, slots));
   CK(dalloc(c->d_facc, 8 * n));  // FP64 forces: 6 words per atom; derivatives: 8
-  CK(dalloc(c->d_cblo, n));
+  CK(dalloc(c->d_cblo, slots));
+  c->slot_room = slots;
   CK(dalloc(c->d_cbhi, n));
   CK(dalloc(c->d_hpos, 3 * n));
   CK(dalloc(c->d_hfrc, 3 * n + kPinOut + 3));  // forces, then the results (pmb200_eval)
@@ -1119,10 +1122,11 @@ int col_prepare(pmb200_ctx *c) {
   }
   g.ncol = g.ncx * g.ncy;
   g.nsz = std::max(1, std::min(kColMaxSlabs, (int)std::lround(L[2] / (0.3 * side))));
-  // buckets of 32 times the mean column, 128 bytes an atom: an unevenly filled box
-  // has long columns (41k atoms of water in three times their edge 12 times the mean;
-  // with twice the mean the sort took 800 us there, 7 in the full box)
-  g.cap = (int)std::min<long long>(n, std::max(2LL * n / g.ncol + 64, 32LL * n / g.ncol));
+  // buckets of twice the mean column, or 32 times, 128 bytes an atom, where reading
+  // the whole list instead takes long: an unevenly filled box has long columns (41k
+  // atoms of water in three times their edge 12 times the mean, in six times 50, where
+  // the overfull columns cost 30 us of 119)
+  g.cap = (int)std::min<long long>(n, (n < 8192 ? 2LL : 32LL) * n / g.ncol + 64);
   g.inv_hs = (float)(g.nsz * u / L[2]);
   g.rc2 = (float)(rlist * rlist / (u * u));
   g.inv_unit = 1.0 / u;
@@ -1135,7 +1139,7 @@ int col_prepare(pmb200_ctx *c) {
   g.nparts = cl >= 16000 ? 1 : (cl >= 2500 ? 2 : (cl >= 600 ? 4 : 8));
   for (c->col_lsplit = 0; 2 << c->col_lsplit <= g.nparts;) c->col_lsplit++;
   c->cg = g;
-  // buffers: the cell kernels' where they are large enough, the rest carved from
+  // buffers: the other kernels' where they are large enough, the rest carved from
   // one allocation (a batch's hundreds of contexts would otherwise spend their
   // construction in the allocator)
   const bool room = (size_t)g.nslot <= c->slot_room;
@@ -1146,14 +1150,17 @@ int col_prepare(pmb200_ctx *c) {
   c->d_cspos = reinterpret_cast<int4 *>(c->d_spos32);
   c->d_cspos64 = c->d_spos64;
   c->d_cw = reinterpret_cast<double4 *>(c->d_rel_lo);
+  c->d_csmeta = reinterpret_cast<int4 *>(c->d_cblo);
+  c->d_csq = reinterpret_cast<double *>(c->d_smeta);
+  c->d_cscratch = c->d_tmp;
+  c->d_icom = reinterpret_cast<int4 *>(c->d_com);
   c->d_cpartial = c->d_partial;
-  // The tables come first, in kTables copies used in turn: an evaluation queued
-  // before this call still reads its own (its other arrays are next written by
-  // work that follows it on its stream).  After the last copy the arena is
-  // allocated anew, and freeing the old one waits for what runs on it.
-  constexpr int kTables = 16;
+  // The counts come first, then the tables in `copies` copies used in turn: an
+  // evaluation queued before this call still reads its own (its other arrays are
+  // next written by work that follows it on its stream).  After the last copy the
+  // arena is allocated anew, and freeing the old one waits for what runs on it.
   const size_t t2 = (size_t)c->ntypes * c->ntypes;
-  const int copies = t2 > 256 ? 1 : kTables;
+  const int copies = t2 > 256 ? 1 : 8;
   auto carve = [&](char *base, int copy) {
     size_t off = 0;
     auto take = [&](auto *&p, size_t count) {
@@ -1161,6 +1168,7 @@ int col_prepare(pmb200_ctx *c) {
       if (base) p = reinterpret_cast<T *>(base + off);
       off = (off + sizeof(T) * count + 255) & ~(size_t)255;
     };
+    take(c->d_ccount, c->col_ncol_alloc);
     for (int k = 0; k < copies; k++) {
       char *const b = base;
       if (k != copy) base = nullptr;
@@ -1175,33 +1183,29 @@ int col_prepare(pmb200_ctx *c) {
       take(c->d_cspos, (size_t)g.nslot);
       take(c->d_cspos64, (size_t)g.nslot);
       take(c->d_cw, (size_t)g.nslot);
+      take(c->d_csmeta, (size_t)g.nslot);
+      take(c->d_csq, (size_t)g.nslot);
+      take(c->d_cscratch, (size_t)g.nslot);
     }
-    take(c->d_csmeta, (size_t)g.nslot);
-    take(c->d_cscratch, (size_t)g.nslot);
-    take(c->d_csq, (size_t)g.nslot);
     take(c->d_bucket, (size_t)g.ncol * g.cap);
     take(c->d_zs, (size_t)g.ncol * (g.nsz + 1));
     take(c->d_csums, g.ncol >= kColScan ? (size_t)g.ncol : 0);
     if (!rows) take(c->d_cpartial, (size_t)c->col_clusters * g.nparts * kNacc);
-    take(c->d_icom, (size_t)std::max(c->nmol, 1));
     return off;
   };
+  const bool more = (size_t)g.ncol > c->col_ncol_alloc;
+  if (more) c->col_ncol_alloc = (size_t)g.ncol;
   const size_t want = carve(nullptr, 0);
-  if (want > c->carena_bytes || ++c->col_tables >= copies) {
+  if (more || want > c->carena_bytes || ++c->col_tables >= copies) {
     const size_t bytes = std::max(want, c->carena_bytes);
     c->carena_bytes = 0;
     CK(dalloc(c->d_carena, bytes));
     c->carena_bytes = bytes;
     c->col_tables = 0;
+    c->col_count_zero = false;
   }
   carve(c->d_carena, c->col_tables);
   // (the counts keep their place: every evaluation leaves them zero)
-  if (c->col_ncol_alloc < (size_t)g.ncol) {
-    c->col_ncol_alloc = 0;
-    CK(dalloc(c->d_ccount, (size_t)g.ncol));
-    c->col_ncol_alloc = (size_t)g.ncol;
-    c->col_count_zero = false;
-  }
   if (!c->col_count_zero) {
     CK(cudaMemsetAsync(c->d_ccount, 0, sizeof(int) * c->col_ncol_alloc, c->stream));
     c->col_count_zero = true;
@@ -1684,7 +1688,7 @@ int pmb200_destroy(pmb200_ctx *c) {
   dfree(c->d_sc_clo); dfree(c->d_sc_chi); dfree(c->d_sc_sbox); dfree(c->d_sc_corg);
   dfree(c->d_sc_sorg); dfree(c->d_sc_tasks); dfree(c->d_sc_cmol); dfree(c->d_sc_ent);
   dfree(c->d_sc_facc); dfree(c->d_sc_part);
-  dfree(c->d_carena); dfree(c->d_ccount);
+  dfree(c->d_carena);
   if (c->h_pin_pos) cudaFreeHost(c->h_pin_pos);
   if (c->h_pin_frc) cudaFreeHost(c->h_pin_frc);
   if (c->h_pin_out) cudaFreeHost(c->h_pin_out); dfree(c->d_hpos); dfree(c->d_hfrc);
@@ -1794,6 +1798,8 @@ int pmb200_set_topology(pmb200_ctx *c, int n, const int *type, const double *q_s
   if (!ex.empty())
     CK(cudaMemcpy(c->d_ex, ex.data(), sizeof(int2) * ex.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->d_mstart, mstart.data(), sizeof(int) * (nmol + 1), cudaMemcpyHostToDevice));
+  c->h_ex_start = std::move(ex_start);
+  c->h_ex = std::move(ex);
   int rc = ensure_atom_buffers(c);
   if (rc) return rc;
   c->have_topo = true;
@@ -3993,36 +3999,47 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
     cuda(cudaMemcpy(b->d_type + a0, c->d_type, sizeof(int) * n, cudaMemcpyDeviceToDevice));
     cuda(cudaMemcpy(b->d_mol + a0, c->d_mol, sizeof(int) * n, cudaMemcpyDeviceToDevice));
     cuda(cudaMemcpy(b->d_q + a0, c->d_q, sizeof(double) * n, cudaMemcpyDeviceToDevice));
-    std::vector<int> es(n + 1);
-    cuda(cudaMemcpy(es.data(), c->d_ex_start, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-    std::vector<int2> e(std::max(es[n], 1));
-    if (es[n] > 0)
-      cuda(cudaMemcpy(e.data(), c->d_ex, sizeof(int2) * es[n], cudaMemcpyDeviceToHost));
     const int base = (int)ex.size();
-    for (int i = 0; i < n; i++) ex_start[a0 + i] = base + es[i];
-    for (int k = 0; k < es[n]; k++) ex.push_back(make_int2(e[k].x + a0, e[k].y));
+    for (int i = 0; i < n; i++) ex_start[a0 + i] = base + c->h_ex_start[i];
+    for (const int2 &e : c->h_ex) ex.push_back(make_int2(e.x + a0, e.y));
   }
   ex_start[N] = (int)ex.size();
   if (rc) return done(rc);
-  cuda(dalloc(b->d_sys, (size_t)nsys));
+  // the column kernels' part (systems that all take them), or the cell kernels'
+  b->col = N > 0;
+  for (int s = 0; s < nsys; s++) b->col = b->col && (systems[s]->col_ok || systems[s]->n == 0);
+  if (b->col) {
+    rc = batch_create_columns(b, systems);
+    if (rc) return done(rc);
+  }
+  if (!b->col) {
+    cuda(dalloc(b->d_sys, (size_t)nsys));
+    cuda(dalloc(b->d_st, std::max<size_t>(st.size(), 1)));
+    cuda(dalloc(b->d_lj32, std::max<size_t>(lj.size(), 1)));
+    cuda(dalloc(b->d_cell_of, n1));
+    cuda(dalloc(b->d_slot, n1));
+    cuda(dalloc(b->d_tmp, n1));
+    cuda(dalloc(b->d_rel32, n1));
+    cuda(dalloc(b->d_spos32, n1));
+    cuda(dalloc(b->d_rel_lo, n1));
+    cuda(dalloc(b->d_spos_lo, n1));
+    cuda(dalloc(b->d_smeta, n1));
+    cuda(dalloc(b->d_count, (size_t)std::max<long long>(C, 1)));
+    cuda(dalloc(b->d_start, (size_t)C + 1));
+    if (rc) return done(rc);
+    cuda(cudaMemcpy(b->d_sys, b->h_sys.data(), sizeof(BatchSys) * nsys, cudaMemcpyHostToDevice));
+    if (!st.empty())
+      cuda(cudaMemcpy(b->d_st, st.data(), sizeof(unsigned short) * st.size(),
+                      cudaMemcpyHostToDevice));
+    if (!lj.empty())
+      cuda(cudaMemcpy(b->d_lj32, lj.data(), sizeof(float4) * lj.size(), cudaMemcpyHostToDevice));
+  }
   cuda(dalloc(b->d_atom_sys, n1));
   cuda(dalloc(b->d_ex_start, n1 + 1));
   cuda(dalloc(b->d_ex, std::max<size_t>(ex.size(), 1)));
-  cuda(dalloc(b->d_st, std::max<size_t>(st.size(), 1)));
-  cuda(dalloc(b->d_lj32, std::max<size_t>(lj.size(), 1)));
-  cuda(dalloc(b->d_cell_of, n1));
-  cuda(dalloc(b->d_slot, n1));
-  cuda(dalloc(b->d_tmp, n1));
   cuda(dalloc(b->d_sidx, n1));
-  cuda(dalloc(b->d_rel32, n1));
-  cuda(dalloc(b->d_spos32, n1));
-  cuda(dalloc(b->d_rel_lo, n1));
-  cuda(dalloc(b->d_spos_lo, n1));
-  cuda(dalloc(b->d_smeta, n1));
   cuda(dalloc(b->d_facc, 3 * n1));
   cuda(dalloc(b->d_scratch_f, 3 * n1));
-  cuda(dalloc(b->d_count, (size_t)std::max<long long>(C, 1)));
-  cuda(dalloc(b->d_start, (size_t)C + 1));
   cuda(dalloc(b->d_err, 1));
   cuda(dalloc(b->d_counter, 1));
   cuda(dalloc(b->d_pairs, (size_t)nsys));
@@ -4030,16 +4047,11 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
   cuda(cudaEventCreate(&b->ev0));
   cuda(cudaEventCreate(&b->ev1));
   if (rc) return done(rc);
-  cuda(cudaMemcpy(b->d_sys, b->h_sys.data(), sizeof(BatchSys) * nsys, cudaMemcpyHostToDevice));
   if (N > 0)
     cuda(cudaMemcpy(b->d_atom_sys, atom_sys.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
   cuda(cudaMemcpy(b->d_ex_start, ex_start.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
   if (!ex.empty())
     cuda(cudaMemcpy(b->d_ex, ex.data(), sizeof(int2) * ex.size(), cudaMemcpyHostToDevice));
-  if (!st.empty())
-    cuda(cudaMemcpy(b->d_st, st.data(), sizeof(unsigned short) * st.size(), cudaMemcpyHostToDevice));
-  if (!lj.empty())
-    cuda(cudaMemcpy(b->d_lj32, lj.data(), sizeof(float4) * lj.size(), cudaMemcpyHostToDevice));
   cuda(cudaMemset(b->d_err, 0, sizeof(int)));
   if (rc) return done(rc);
   // dynamic shared memory: the largest LJ table, then the largest stencil
@@ -4058,12 +4070,8 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
     cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel, 32, b->smem));
     out = std::max(1, o);
   };
-  // the column kernels' part (systems that all take them)
-  b->col = N > 0;
-  for (int s = 0; s < nsys; s++) b->col = b->col && (systems[s]->col_ok || systems[s]->n == 0);
+  // per (energy, virial) variant of the batch's form
   if (b->col) {
-    rc = batch_create_columns(b, systems);
-    if (rc) return done(rc);
     for (int v = 0; v < 4; v++) {
       ColArrays a{};
       const ColBatchLaunch l = batch_col_launch(b, v & 1, v & 2, a);
@@ -4071,9 +4079,6 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
       cuda(col_launch_batch(a, l, nullptr, &o));
       b->occ[v] = std::max(1, o);
     }
-  }
-  // per (energy, virial) variant of the batch's form
-  if (b->col) {
   } else if (b->form == FORM_GENERIC) {
     fits(k_pair_mixed_batch<FORM_GENERIC, false, false>, b->occ[0]);
     fits(k_pair_mixed_batch<FORM_GENERIC, true, false>, b->occ[1]);
