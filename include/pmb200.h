@@ -150,30 +150,33 @@ int pmb200_eval_cells(pmb200_ctx *ctx, const double *pos, double *forces,
 int pmb200_eval_device(pmb200_ctx *ctx, const double *d_pos, double *d_forces,
                        double *d_out, unsigned flags, void *stream);
 
-/* Autotuner of one context's evaluation.  Times the whole evaluation (cell
- * build, pair kernel, force finalisation, reductions) on the device
- * positions d_pos[3n], reps timed launches per configuration (median), with
- * and without energies, over the grid's cell size (hints cutoff / 1.5, / 2,
- * / 2.5, / 3, / 3.5, / 4, each as pmb200_params::cellsize; hints that give
- * the same grid are timed once, grids the stencil limits refuse are skipped)
- * and, for PMB200_MIXED contexts, the pair kernel (search or cluster-pair,
- * see pmb200_set_pair_kernel) and its warps per i-cell (2, 4, 8), chosen
- * separately for energy launches and forces-only launches, then the
- * supercluster kernel on the chosen grid where it applies; keeps the grid
- * with the fastest evaluation with energies (the reference's integrators
- * ask for energies every step) and applies it.  The library's defaults are
- * timed first and another configuration replaces them only when it is 2%
- * faster (timing noise between near-equal ones does not move the choice).  The choice is cached for the
- * process under a key of the device, the force (kind, precision, cutoffs,
- * switches), the atom and type counts and the box: a later context with the
- * same key takes it without timing.  result[8] (may be NULL) = {cell-size
- * hint, warps per i-cell with energies, warps per i-cell forces-only (0 for
- * FP64), ms with energies, ms forces-only, configurations timed (0: taken
- * from the cache), pair kernel with energies, pair kernel forces-only
- * (PMB200_KERNEL_*)}.  Forces and energies after tuning agree with the
- * untuned ones to the kernel's precision (the cell grid sets the FP32
- * cell-unit coordinates).  The device work runs on `stream` (NULL: the
- * context's) and is synchronised. */
+/* Autotuner of one context's evaluation.  Times the whole evaluation (build,
+ * pair kernel, force finalisation, reductions) on the device positions
+ * d_pos[3n], reps timed launches per configuration (median), with and without
+ * energies.  Configurations:
+ *  - the search (see pmb200_set_pair_kernel): where the column kernels are it,
+ *    which take neither a cell size nor warps per i-cell, one;
+ *  - elsewhere the cell kernels over the grid's cell size (hints cutoff / 1.5,
+ *    / 2, / 2.5, / 3, / 3.5, / 4, each as pmb200_params::cellsize; hints that
+ *    give the same grid are timed once, grids the stencil limits refuse are
+ *    skipped) and, in mixed contexts, the warps per i-cell (2, 4, 8), chosen
+ *    separately for energy launches and forces-only launches;
+ *  - in PMB200_MIXED contexts the cluster-pair kernel over the same grids and
+ *    warps, then the supercluster kernel on the chosen grid, where they apply.
+ * Keeps the configuration with the fastest evaluation with energies (the
+ * reference's integrators ask for energies every step) and applies it.  The
+ * library's defaults are timed first and another configuration replaces them
+ * only when it is 2% faster (timing noise between near-equal ones does not
+ * move the choice).  The choice is cached for the process under a key of the
+ * device, the force (kind, precision, cutoffs, switches), the atom and type
+ * counts and the box: a later context with the same key takes it without
+ * timing.  result[8] (may be NULL) = {cell-size hint, warps per i-cell with
+ * energies, warps per i-cell forces-only (0 for FP64; with the column kernels
+ * both these and the hint are the defaults), ms with energies, ms forces-only,
+ * configurations timed (0: taken from the cache), pair kernel with energies,
+ * pair kernel forces-only (PMB200_KERNEL_*)}.  Forces and energies after tuning
+ * agree with the untuned ones to the kernel's precision.  The device work runs
+ * on `stream` (NULL: the context's) and is synchronised. */
 int pmb200_autotune(pmb200_ctx *ctx, const double *d_pos, void *stream, int reps,
                     double result[8]);
 

@@ -2155,6 +2155,7 @@ int pmb200_autotune(pmb200_ctx *c, const double *d_pos, void *stream, int reps,
       return PMB200_OK;
     };
     int last_dims[3] = {-1, -1, -1};
+    double col_e = 0.0, col_f = 0.0;  // the column kernels' times, once known
     best.ms_e = 1e300;
     int status = PMB200_OK;
     const double *divs = tric0 ? divs_t : divs_o;
@@ -2169,18 +2170,32 @@ int pmb200_autotune(pmb200_ctx *c, const double *d_pos, void *stream, int reps,
       TuneChoice cand{};
       cand.cellsize = c->p.cellsize;
       cand.ms_e = cand.ms_f = 1e300;
-      // the search kernel, and the cluster-pair kernel where it applies
+      // the search kernel, and the cluster-pair kernel where it applies.  The
+      // column kernels, where they are the search, take neither the cell size nor
+      // the warps per i-cell: one timing stands for all grids.
       for (int kern = 0; kern < 2 && !status; kern++) {
         c->tiles_e = c->tiles_f = kern == 1;
         if (kern == 1 && !tiles_apply(c, PMB200_ENERGY) && !tiles_apply(c, 0u)) break;
+        const bool cols = kern == 0 && c->col_ok;
+        if (cols && col_e > 0.0) {
+          cand.ms_e = col_e;
+          cand.ms_f = col_f;
+          cand.slots_e = cand.slots_f = mixed ? slot_opts[0] : 0;
+          continue;
+        }
         for (int so : slot_opts) {
-          if (!mixed && so != slot_opts[0]) break;  // the FP64 kernel's split is fixed
+          // (the FP64 kernel's split is fixed)
+          if ((!mixed || cols) && so != slot_opts[0]) break;
           double me = 0.0, mf = 0.0;
           c->slots_e = c->slots_f = mixed ? so : 0;
           status = timed(PMB200_ENERGY, me);
           if (!status) status = timed(0u, mf);
           if (status) break;
           best.tried++;
+          if (cols) {
+            col_e = me;
+            col_f = mf;
+          }
           if (faster(me, cand.ms_e)) {
             cand.ms_e = me;
             cand.slots_e = mixed ? so : 0;

@@ -282,8 +282,9 @@ class NonbondedCutoffB200SystemForce:
 
     def autotune(self, topo, pos_ptr, reps=10, stream=None):
         """pmb200_autotune on device positions (a raw pointer): times the
-        evaluation over cell sizes and, for mixed precision, warps per i-cell,
-        applies the fastest and returns the choice as a dict."""
+        evaluation over the pair kernels and, where they are cell kernels, over
+        cell sizes and, for mixed precision, warps per i-cell, applies the fastest
+        and returns the choice as a dict."""
         self._ensure(topo)
         r = (ctypes.c_double * 8)()
         self._check(_lib.lib().pmb200_autotune(self._ctx, _P(pos_ptr),

@@ -96,3 +96,28 @@ def test_tuning_on_the_legacy_default_stream():
     from oracle import oracle as O
     fo, eo, _, _ = O.restate_eval(d, d["pos"], virial_mode=0)
     assert rms_rel(F, fo) <= 1e-5
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_the_column_kernels_are_timed_once(precision):
+    """Neither the cell size nor the warps per i-cell reach the column kernels: with
+    more types than the other kernels take they are the one configuration.  In
+    a box too long for them the cell kernels are tuned over their grids."""
+    import torch
+    from protomoladdon_b200 import water
+    d = water.water_box(7, rc=8.0, ron=7.0, seed=22)
+    many = np.zeros((17, 17, 4))
+    many[:2, :2] = d["lj"]
+    d["lj"] = many
+    pos = torch.tensor(d["pos"], dtype=torch.float64, device="cuda:0")
+    for length, once in ((d["box"][2], True), (1300.0, False)):
+        d["box"] = np.array([d["box"][0], d["box"][1], length])
+        f = NonbondedCutoffB200SystemForce(d["ron"], d["rc_lj"], d["rc_coul"], d["rc_alg"],
+                                           precision=precision)
+        choice = f.autotune(PeriodicTopology.from_dict(d), pos.data_ptr(), reps=2)
+        f.close()
+        assert choice["kernel_energy"] == choice["kernel_forces"] == "search"
+        assert (choice["configurations_timed"] == 1) == once
+        if once:
+            assert choice["cellsize_hint"] == d["rc_alg"] / 2.0
+            assert choice["warps_per_cell_energy"] == (4 if precision == "mixed" else 0)
