@@ -24,7 +24,8 @@ from oracle import oracle as O
 from protomoladdon_b200 import _lib, water
 from protomoladdon_b200.autograd import NonbondedEnergy
 from protomoladdon_b200.batch import SystemBatch
-from protomoladdon_b200.force import (NonbondedCutoffB200SystemForce, PeriodicTopology,
+from protomoladdon_b200.force import (EwaldRealB200SystemForce, NonbondedCutoffB200PairForce,
+                                      NonbondedCutoffB200SystemForce, PeriodicTopology,
                                       ScalarStructure)
 
 pytestmark = pytest.mark.gpu
@@ -226,3 +227,138 @@ def test_batch_against_oracle():
             assert np.sqrt(((got - fo) ** 2).sum()) <= 1e-5 * max(np.sqrt((fo ** 2).sum()), 1e-30)
             assert np.abs(out[k, :2].cpu().numpy() - eo[:2]).max() <= 1e-4 * s["n"]
     b.close()
+
+
+FORM_CASES = ["one_water", "two_cutoffs", "odd_edges_unwrapped", "dilute_tall_clusters",
+              "long_exclusion_lists", "modified_pairs", "tall_block_in_vacuum"]
+
+
+def _form(form, s, precision):
+    """A force of the form, and the oracle's forces, energies, virials and pairs."""
+    rc = s["rc_coul"]
+    if form in ("poly5", "exact"):
+        alpha, acc = 3.0 / rc, float(np.exp(-9.0))
+        fo, eo, vo, mo = O.restate_ewald_real(s, s["pos"], alpha, acc, form == "exact", 2)
+        return (EwaldRealB200SystemForce(alpha, acc, precision=precision, erfc=form), fo,
+                np.array([eo, 0.0]), vo, mo)
+    fo, eo, vo, mo = O.restate_eval(s, s["pos"], virial_mode=2)
+    if form == "switches":  # the same potential through the general switches
+        f = NonbondedCutoffB200PairForce(("C2", s["ron"], rc), ("C1", 0.0, rc), rc,
+                                         precision=precision)
+    else:
+        f = NonbondedCutoffB200SystemForce(s["ron"], rc, rc, rc, precision=precision)
+    return f, fo, np.asarray(eo), vo, mo
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("form", ["poly5", "exact", "switches", "many_types"])
+@pytest.mark.parametrize("name", FORM_CASES)
+def test_forms_against_oracle(name, form, precision):
+    """The other forms and tables beyond shared memory at the same edges; with the
+    general switches energies to 1e-6 of the unswitched pair magnitudes, about
+    1,000 kcal/mol per atom."""
+    s = CASES[name]()
+    if form == "many_types":
+        s = water.many_types(s)
+    f, fo, eo, vo, mo = _form(form, s, precision)
+    topo = PeriodicTopology.from_dict(s)
+    F, E = np.zeros_like(s["pos"]), ScalarStructure()
+    f.evaluate(topo, s["pos"], F, E)
+    Fv, Ev = np.zeros_like(F), ScalarStructure(virial=True, molecular_virial=True)
+    f.evaluate(topo, s["pos"], Fv, Ev)
+    f.close()
+    tol, etol = (1e-5, 1e-3 if form == "switches" else 1e-4) if precision == "mixed" else (1e-12,
+                                                                                         1e-9)
+    for got, e in ((F, E), (Fv, Ev)):
+        assert np.sqrt(((got - fo) ** 2).sum()) <= tol * max(np.sqrt((fo ** 2).sum()), 1e-30)
+        assert max(abs(e[0] - eo[0]), abs(e[1] - eo[1])) <= etol * s["n"]
+    for got, want in ((Ev.virial_matrix(), vo), (Ev.molvirial_matrix(), mo)):
+        want = np.asarray(want).reshape(3, 3)
+        assert np.abs(got - want).max() <= 1e-5 * max(np.abs(want).max(), 1.0)
+
+
+@pytest.mark.parametrize("name", ["tall_block_in_vacuum", "thread_in_vacuum", "two_cutoffs"])
+def test_shares_sum_to_one_evaluation(name):
+    """Shards (bit for bit) and cell ranges (host sums) on overfull layouts."""
+    s = CASES[name]()
+    topo = PeriodicTopology.from_dict(s)
+    f = NonbondedCutoffB200SystemForce(s["ron"], s["rc_lj"], s["rc_coul"], s["rc_alg"])
+    pos = torch.tensor(s["pos"], device="cuda")
+    frc = torch.zeros_like(pos)
+    out = torch.zeros(20, dtype=torch.float64, device="cuda")
+    f.evaluate_device(topo, pos.data_ptr(), frc.data_ptr(), out.data_ptr(), _lib.PMB200_ENERGY, 1)
+    total = torch.zeros(3 * s["n"], dtype=torch.int64, device="cuda")
+    for k in range(3):
+        facc = torch.full_like(total, 12345)  # (overwritten)
+        f.shard_eval_device(topo, pos.data_ptr(), k, 3, facc.data_ptr(), None, 0, 1)
+        total += facc
+    sharded = torch.zeros_like(pos)
+    f.shard_finalize(total.data_ptr(), sharded.data_ptr(), 1)
+    torch.cuda.synchronize()
+    want = frc.cpu().numpy()
+    scale = np.abs(want).max()
+    # (a launch without energies takes the same pairs in the same groups)
+    assert np.abs(sharded.cpu().numpy() - want).max() <= 1e-6 * scale
+    blocks = f.number_of_blocks(topo)
+    F, E = np.zeros_like(want), ScalarStructure()
+    for lo, hi in ((0, blocks // 3), (blocks // 3, blocks // 2), (blocks // 2, blocks)):
+        f.evaluate_cells(topo, s["pos"], F, E, lo, hi)
+    f.close()
+    assert np.abs(F - want).max() <= 1e-12 * scale
+    e = out.cpu().numpy()
+    assert max(abs(E[0] - e[0]), abs(E[1] - e[1])) <= 1e-12 * max(abs(e[0]), abs(e[1]), 1.0)
+
+
+def _derivatives(s, v, padded):
+    """H v and the parameter derivatives of E and of v . G; padded: five types in the
+    table, which the general derivative kernel serves."""
+    s = dict(s)
+    nt = len(s["lj"])
+    if padded:
+        lj = np.zeros((5, 5, 4))
+        lj[:nt, :nt] = s["lj"]
+        s["lj"] = lj
+    m = NonbondedEnergy.from_system(s, precision="fp64")
+    q, t = (x.requires_grad_(True) for x in m.initial_params())
+    pos = torch.tensor(s["pos"], device="cuda", requires_grad=True)
+    first = torch.autograd.grad(m.energy(pos, q, t), (q, t))
+    g = m.gradient(pos, q, t)
+    second = torch.autograd.grad(g, (pos, q, t), grad_outputs=torch.tensor(v, device="cuda"))
+    m.force.sync()
+    m.close()
+    cut = lambda x: x[:nt, :nt] if x.dim() == 3 else x  # noqa: E731
+    return [cut(x.detach()).cpu().numpy() for x in first + second]
+
+
+@pytest.mark.parametrize("name", HVP_CASES)
+def test_derivatives_against_the_general_kernel(name):
+    """Products and parameter derivatives on the column walk, modified pairs among
+    them, against the cell walk that serves larger tables: the same FP64 terms in
+    another order."""
+    s = CASES[name]()
+    v = _direction(s)
+    for a, b in zip(_derivatives(s, v, False), _derivatives(s, v, True)):
+        assert np.linalg.norm(a - b) <= 1e-12 * max(np.linalg.norm(b), 1e-30)
+
+
+def test_a_direction_that_is_not_finite_stays_local():
+    """A NaN in the direction reaches the products of the atoms within the cutoff of
+    its atom, and no others."""
+    s = CASES["odd_edges_unwrapped"]()
+    m = NonbondedEnergy.from_system(s, precision="fp64")
+    q, t = m.initial_params()
+    pos = torch.tensor(s["pos"], device="cuda", requires_grad=True)
+    g = m.gradient(pos, q, t)
+    v = torch.tensor(_direction(s), device="cuda")
+    (want,) = torch.autograd.grad(g, pos, grad_outputs=v, retain_graph=True)
+    m.force.sync()
+    bad = v.clone()
+    bad[7, 1] = float("nan")
+    (got,) = torch.autograd.grad(g, pos, grad_outputs=bad)
+    with pytest.raises(_lib.PmbError):
+        m.force.sync()
+    m.close()
+    d = s["pos"] - s["pos"][7]
+    d -= s["box"] * np.rint(d / s["box"])
+    far = torch.tensor(np.sqrt((d ** 2).sum(1)) > s["rc_coul"] + 1e-6, device="cuda")
+    assert torch.equal(got[far], want[far]) and far.sum() > s["n"] // 4
