@@ -1135,6 +1135,15 @@ int col_prepare(pmb200_ctx *c) {
   const long long slots = (long long)n + (long long)(kColI - 1) * std::min(n, g.ncol);
   g.nslot = (int)((slots + kColI - 1) / kColI * kColI);
   c->col_clusters = g.nslot / kColI;
+  // Parts of a cluster's neighbour columns, a warp each: enough warps for the chip
+  // against one more partly filled block of 32 and search set-up per part.  Water,
+  // rc 10, forces (us) with 1 / 2 / 4 / 8 parts: 648 atoms 29 / 27 / 27 / 28, 2,400
+  // 43 / 31 / 27 / 28, 6,000 45 / 35 / 33 / 35, 15,009 66 / 51 / 51 / 57, 41,472 90 /
+  // 90 / 98 / 121, 123,000 213 / 221 / 254 / 324, 332k 498 / 532 / 621 / 815;
+  // energies the same way (41,472: 119 / 121 / 133 / 168), FP64 forces 43 / 33 / 27 /
+  // 28 at 648, 80 / 75 / 70 / 77 at 15,009 and 131 / 133 / 141 / 172 at 41,472,
+  // Hessian-vector products 53 / 37 / 29 / 28, 97 / 94 / 94 / 107 and 203 / 193 / 207 /
+  // 252.  One rule for all, so that an evaluation and a batch group their sums alike.
   const int cl = n / kColI;
   g.nparts = cl >= 16000 ? 1 : (cl >= 2500 ? 2 : (cl >= 600 ? 4 : 8));
   for (c->col_lsplit = 0; 2 << c->col_lsplit <= g.nparts;) c->col_lsplit++;

@@ -1124,7 +1124,7 @@ __device__ __forceinline__ void col_task(const ColGrid &g, const MixedConsts &mc
 
 // One warp per block, each its own task (a warp that finishes early frees its
 // slot): block b takes cluster b >> lsplit, parts (b & (2^lsplit - 1)) + k 2^lsplit.
-// [lo, hi) of `of`: the clusters [total lo / of, total hi / of).
+// share: the part of the clusters that this launch takes.
 // Dynamic shared memory: the warp's entries, then the LJ tables (for exact
 // energies double2 {A, B} [and {A14, B14}], float4; up to kMaxTypes types).
 #ifndef PMB200_COL_BLOCKS

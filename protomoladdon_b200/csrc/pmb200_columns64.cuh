@@ -69,11 +69,11 @@ struct ColWalk64 {
   Pair &pair;
   int nl = 0, nn = 0;  // staged entries from the front, from the back
 
-  template <class Tag>
   // half: the block's first 16 entries, four per lane group -- two lanes then
   // meet one entry, each with its own part of the j terms, and four steps are
   // enough (3% of the derivative kernels' time; the mixed kernel, with shorter
   // steps, lost as much to the choice as it gained)
+  template <class Tag>
   __device__ __forceinline__ void block(Tag tag, int e0, bool half) {
     const int lane = threadIdx.x & 31;
     const unsigned e = (unsigned)(e0 + (half ? 4 * (lane >> 3) + (lane & 3) : lane));
@@ -361,10 +361,15 @@ struct ColPair64 {
   }
 };
 
+// (41,472 atoms, forces / with energies at 14, 16, 18, 20, 22, 24 blocks: 139 / 148,
+// 141 / 149, 129 / 139, 133 / 139, 125 / 133, 125 / 133 us)
 #ifndef PMB200_COL64_BLOCKS
 #define PMB200_COL64_BLOCKS 20
 #endif
-constexpr int kCol64LjTypes = 8;  // LJ tables up to this size in shared memory
+// LJ tables up to this size in shared memory (forces of 41,472 atoms with 4, 8, 12
+// and 16 types: 145, 148, 150 and 166 us from shared memory, where large tables
+// cost residency, 145, 146, 148 and 149 through L1)
+constexpr int kCol64LjTypes = 8;
 
 // (launch, clusters and parts as k_col_pair; dynamic shared memory: the entries,
 // then the LJ table)
@@ -534,6 +539,9 @@ struct ColDeriv64 {
   }
 };
 
+// (a product of 41,472 atoms at 12, 14, 16, 18, 20 blocks 213, 189, 193, 178, 178 us;
+// dE/dparams at 8, 10, 12, 14, 16 blocks 234, 234, 233, 199, 199, both together 420,
+// 326, 322, 285, 285)
 #ifndef PMB200_COLD_BLOCKS
 #define PMB200_COLD_BLOCKS 16
 #endif
