@@ -106,7 +106,9 @@ int pmb200_set_topology(pmb200_ctx *ctx, int n, const int *type,
  * differences rounded to the nearest lattice vector); the distance between
  * opposite faces must be about 3 cutoffs or more (each axis must hold
  * 2 ceil(rc / cell width) + 1 cells of at least rc / 4; PMB200_EUNSUPPORTED
- * otherwise).  Batches take orthogonal boxes only. */
+ * otherwise).  Batches take orthogonal boxes only.  Evaluations already queued
+ * keep the box they were queued with; a caller's own graph of evaluations holds
+ * the box and the buffers of its capture and is captured anew after this call. */
 int pmb200_set_box(pmb200_ctx *ctx, const double e1[3], const double e2[3],
                    const double e3[3], const double origin[3]);
 
