@@ -117,6 +117,7 @@ struct pmb200_ctx {
   bool have_topo = false, have_box = false, have_mass = false;
   double csf = 1.0;
   std::vector<double> h_lj;  // ntypes^2 * 4
+  std::vector<int> h_ntype;  // atoms of each type
   std::vector<int> h_ex_start;  // the exclusion lists of d_ex_start and d_ex (batches)
   std::vector<int2> h_ex;
   int *d_type = nullptr, *d_mol = nullptr;
@@ -1077,14 +1078,25 @@ int col_prepare(pmb200_ctx *c) {
     g.q[a] = (float)g.qd[a];
   }
   // columns about the edge of a cube of kColI atoms wide (measured on water:
-  // 0.9 to 1.15 times that edge within 2%), slabs 0.3 of it high.  At most
-  // kColMaxSide cutoffs, since the mean density says little of a box that is not
-  // uniformly filled: 41k atoms of water in a cube of 3, 4 and 6 times their edge
+  // 0.9 to 1.15 times that edge within 2%), slabs 0.3 of it high.  The mean density
+  // says little of a box that is not uniformly filled, so the width is at most
+  // kColMaxSide cutoffs: 41k atoms of water in a cube of 3, 4 and 6 times their edge
   // take 88, 88 and 119 us (forces) so, 106, 106 and 135 with one cutoff, 137, 185 and
   // 201 with 1.4; filled 90.  A gas of 1/216 of water's density, 41k atoms, takes 45,
-  // 41 and 35 us.
+  // 41 and 35 us.  Short cutoffs are left the edge of a cube of kColI atoms packed at
+  // their Lennard-Jones volume sigma^3 = sqrt(A / B) (4.4 A in water): a filled box of
+  // 332k atoms takes 125, 137 and 152 us at rc 2.5, 3 and 4 so, 174, 168 and 164 if
+  // held to kColMaxSide cutoffs.
+  int r = pull_lj(c);
+  if (r) return r;
+  double volume = 0.0;
+  for (int t = 0; t < c->ntypes; t++) {
+    const double *p = &c->h_lj[4 * ((size_t)t * c->ntypes + t)];
+    if (p[0] > 0.0 && p[1] > 0.0) volume += c->h_ntype[t] * std::sqrt(p[0] / p[1]);
+  }
   const double rlist = rc * (1.0 + 1e-5);
-  double side = std::min(std::cbrt(kColI * L[0] * L[1] * L[2] / n), kColMaxSide * rc);
+  double side = std::min(std::cbrt(kColI * L[0] * L[1] * L[2] / n),
+                         std::max(kColMaxSide * rc, std::cbrt(kColI * volume / n)));
   for (;; side *= 1.25) {
     g.ncx = std::max(1, std::min(16384, (int)std::lround(L[0] / side)));
     g.ncy = std::max(1, std::min(16384, (int)std::lround(L[1] / side)));
@@ -1221,8 +1233,6 @@ int col_prepare(pmb200_ctx *c) {
   }
   c->mcc = mixed_consts(c, rc, u);
   c->col_full = c->mcc.rclj2 >= c->mcc.cut2 && c->mcc.rcc2 >= c->mcc.cut2;
-  int r = pull_lj(c);
-  if (r) return r;
   r = col_upload(c);
   if (r) return r;
   c->col_ok = true;
@@ -1783,6 +1793,8 @@ int pmb200_set_topology(pmb200_ctx *c, int n, const int *type, const double *q_s
   c->have_mass = mass != nullptr;
   c->col_ok = false;  // (until prepare_kernels; the tables' sizes change)
   c->h_lj.assign(lj, lj + 4 * ntypes * ntypes);
+  c->h_ntype.assign((size_t)ntypes, 0);
+  for (int i = 0; i < n; i++) c->h_ntype[type[i]]++;
   c->lj_dev_newer = false;
   const size_t nn = (size_t)std::max(n, 1);
   CK(dalloc(c->d_type, nn));

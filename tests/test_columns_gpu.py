@@ -111,6 +111,7 @@ CASES = {
     "tall_block_in_vacuum": lambda: _waters(727, (150.0, 140.0, 400.0), (11.0, 11.0, 180.0)),
     "thread_in_vacuum": lambda: _waters(1540, (52.5, 52.5, 1250.0), (6.2, 6.2, 1197.0), rc=11.0),
     "many_columns": lambda: _waters(4500, (1000.0, 1000.0, 16.5), (300.0, 300.0, 16.5)),
+    "short_cutoff": lambda: _waters(400, (40.0, 23.0, 40.0), (22.0, 23.0, 24.0), rc=3.0),
     "full_last_flush_104_37": lambda: _ball(104, 37),
     "full_last_flush_99_5": lambda: _ball(99, 5),
     "full_last_flush_104_95": lambda: _ball(104, 95),
