@@ -185,8 +185,8 @@ int pmb200_autotune(pmb200_ctx *ctx, const double *d_pos, void *stream, int reps
 /* The mixed pair kernel of a context.  PMB200_KERNEL_SEARCH (the default):
  * a search in every evaluation -- on orthogonal periodic boxes the column
  * kernels (clusters of 8 atoms against the atoms within the cutoff of their
- * box), elsewhere and where an edge exceeds 160 cutoffs (the column kernels
- * hold coordinates to 2^-32 of the edge) per-atom candidate search (culled
+ * box), elsewhere and where an edge exceeds 160 cutoffs (the mixed column
+ * kernels hold coordinates to 2^-32 of the edge) per-atom candidate search (culled
  * staging, per-lane lists).  PMB200_KERNEL_TILES: cluster pairs -- runs of 4
  * atoms of a cell (sorted by height) as clusters, one bounding-box test per
  * cluster pair, and 4 x 4 tiles of atom pairs evaluated with masks; the same pair set and

@@ -79,7 +79,7 @@ struct pmb200_ctx {
   double *d_sc_part = nullptr;
   // column kernels (pmb200_columns.cuh), where they apply (col_ok): the
   // evaluation path of orthogonal periodic boxes
-  bool col_ok = false, col_full = false;
+  bool col_ok = false, col_mixed = false, col_full = false;  // (col_mixed: to the mixed ones)
   ColGrid cg{};
   ColStencil cst{};
   short2 *d_cst = nullptr;    // its classes on the device
@@ -1045,7 +1045,8 @@ int launch_eval_clusters(pmb200_ctx *c, const double *d_pos, double *d_forces, d
   return PMB200_OK;
 }
 
-constexpr double kColMaxEdge = 160.0;  // box edge, in cutoffs (see col_prepare)
+constexpr double kColMaxEdge = 160.0;    // box edge, in cutoffs (see col_prepare):
+constexpr double kColMaxEdge64 = 4096.0; // mixed and FP64 kernels
 constexpr double kColMaxSide = 0.7;    // column width, in cutoffs
 
 // The column kernels' grid, neighbour columns, constants, tables and buffers
@@ -1058,13 +1059,17 @@ int col_prepare(pmb200_ctx *c) {
   const int n = c->n;
   const double rc = ctx_rc(c);
   const double *L = c->g.boxlen;
-  // a coordinate is held to 2^-32 of its edge.  Water in a box of growing length, RMS
-  // force error and Coulomb energy error per atom (kcal/mol) at rc 9: edges up to
-  // 300 A 7.7e-7, 2e-9; 1,200 A 7.7e-7, 8e-9; 2,400 A 8.2e-7, 2.3e-8; 19,200 A 3.0e-6,
-  // 1.6e-7; the cell kernels (coordinates within a cell) 9.5e-7 and 2e-8 to 6e-8
-  // throughout.  The FP64 kernels' box tests need edges below some 20,000 rc.
-  for (int a = 0; a < 3; a++)
-    if (L[a] > kColMaxEdge * rc) return PMB200_OK;
+  // a coordinate is held to 2^-32 of its edge.  Mixed evaluations are made of these:
+  // water in a box of growing length, RMS force error and Coulomb energy error per
+  // atom (kcal/mol) at rc 9: edges up to 300 A 7.7e-7, 2e-9; 1,200 A 7.7e-7, 8e-9;
+  // 2,400 A 8.2e-7, 2.3e-8; 19,200 A 3.0e-6, 1.6e-7; the cell kernels (coordinates
+  // within a cell) 9.5e-7 and 2e-8 to 6e-8 throughout.  The FP64 kernels only search
+  // with them: two quanta, here 2e-6 cutoffs, against the box tests' margin of 1e-5.
+  c->col_mixed = true;
+  for (int a = 0; a < 3; a++) {
+    if (L[a] > kColMaxEdge64 * rc) return PMB200_OK;
+    c->col_mixed = c->col_mixed && L[a] <= kColMaxEdge * rc;
+  }
   ColGrid g{};
   // lengths in units of a power-of-two fraction of the x edge (about 4 A): one
   // quantum is then an exact FP32 number along x, and along y and z in cubes
@@ -1248,7 +1253,7 @@ int prepare_kernels(pmb200_ctx *c) {
 // Whether an evaluation runs on the column kernels: where they apply and no
 // other pair kernel was asked for (and serves it).
 bool columns_apply(const pmb200_ctx *c, unsigned flags) {
-  return c->col_ok && c->p.precision == PMB200_MIXED && !clusters_apply(c, flags) &&
+  return c->col_ok && c->col_mixed && c->p.precision == PMB200_MIXED && !clusters_apply(c, flags) &&
          !tiles_apply(c, flags);
 }
 
@@ -2197,7 +2202,7 @@ int pmb200_autotune(pmb200_ctx *c, const double *d_pos, void *stream, int reps,
       for (int kern = 0; kern < 2 && !status; kern++) {
         c->tiles_e = c->tiles_f = kern == 1;
         if (kern == 1 && !tiles_apply(c, PMB200_ENERGY) && !tiles_apply(c, 0u)) break;
-        const bool cols = kern == 0 && c->col_ok;
+        const bool cols = kern == 0 && c->col_ok && (c->col_mixed || !mixed);
         if (cols && col_e > 0.0) {
           cand.ms_e = col_e;
           cand.ms_f = col_f;
@@ -2358,7 +2363,7 @@ int pmb200_shard_eval_device(pmb200_ctx *c, const double *d_pos, int shard, int 
   const int lo = (int)((long long)g.ncell * shard / nshards);
   const int hi = (int)((long long)g.ncell * (shard + 1) / nshards);
   unsigned long long *facc = reinterpret_cast<unsigned long long *>(d_facc);
-  if (c->col_ok) {
+  if (c->col_ok && c->col_mixed) {
     rc = launch_col_build(c, d_pos, st, facc, (flags & PMB200_MOLVIRIAL) != 0);
     if (rc) return rc;
     const ColShare share{shard, shard + 1, nshards};
@@ -2413,7 +2418,7 @@ int pmb200_shard_finalize(pmb200_ctx *c, const long long *d_facc, double *d_forc
   CK(cudaSetDevice(c->p.device));
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   const unsigned long long *facc = reinterpret_cast<const unsigned long long *>(d_facc);
-  if (c->n > 0 && c->col_ok)
+  if (c->n > 0 && c->col_ok && c->col_mixed)
     k_col_finalize<false><<<(c->n + 255) / 256, 256, 0, st>>>(
         c->n, facc, c->d_sidx, kFixInv / c->col_unit, 1, d_forces, nullptr);
   else if (c->n > 0)
@@ -2859,7 +2864,7 @@ int pmb200_eval_cells(pmb200_ctx *c, const double *pos, double *forces, double *
   const bool anyvir = (flags & (PMB200_VIRIAL | PMB200_MOLVIRIAL)) != 0;
   const GridParams &g = c->g;
   const int nc = cell_hi - cell_lo;
-  if (mixed && c->col_ok) {
+  if (mixed && c->col_ok && c->col_mixed) {
     // column kernels: the share of the clusters that the range is of the cells
     const ColShare share{cell_lo, cell_hi, g.ncell};
     rc = launch_col_build(c, c->d_hpos, st, c->d_facc, (flags & PMB200_MOLVIRIAL) != 0);
@@ -4043,7 +4048,8 @@ int pmb200_batch_create(pmb200_ctx *const *systems, int nsys, pmb200_batch **out
   if (rc) return done(rc);
   // the column kernels' part (systems that all take them), or the cell kernels'
   b->col = N > 0;
-  for (int s = 0; s < nsys; s++) b->col = b->col && (systems[s]->col_ok || systems[s]->n == 0);
+  for (int s = 0; s < nsys; s++)
+    b->col = b->col && ((systems[s]->col_ok && systems[s]->col_mixed) || systems[s]->n == 0);
   if (b->col) {
     rc = batch_create_columns(b, systems);
     if (rc) return done(rc);

@@ -163,11 +163,13 @@ def test_fp64_against_oracle(name):
 
 @pytest.mark.parametrize("precision,length,tol", [
     ("mixed", 1279.0, 2e-6), ("mixed", 1281.0, 2e-6), ("mixed", 19200.0, 2e-6),
-    ("fp64", 1281.0, 1e-12), ("fp64", 6e5, 1e-12)])
+    ("fp64", 1281.0, 1e-12), ("fp64", 32760.0, 1e-12), ("fp64", 32800.0, 1e-12),
+    ("fp64", 6e5, 1e-12)])
 def test_long_boxes(precision, length, tol):
     """The column kernels hold a coordinate to 2^-32 of its edge (at 19,200 A three
-    times the FP32 force error of about 1e-6): longer boxes run on the cell kernels,
-    with the same errors as short ones."""
+    times the FP32 force error of about 1e-6): mixed evaluations of longer boxes, and
+    FP64 ones from 4,096 cutoffs on, run on the cell kernels, with the same errors as
+    short ones."""
     s = _waters(400, (20.0, 20.0, length), (20.0, 20.0, 30.0), rc=8.0)
     s["pos"] = s["pos"] + np.array([0.0, 0.0, 0.37 * length])
     f = NonbondedCutoffB200SystemForce(s["ron"], s["rc_lj"], s["rc_coul"], s["rc_alg"],
